@@ -913,6 +913,7 @@ PfSolveResult append_jw(PfSolveApplication* app, const PfSolveLaunchParams* lp, 
         op.alt = 1;
         op.alt_T = s->alt_T;
         op.alt_R = s->alt_R;
+        op.alt_mul = fast_div_mul(s->alt_R);
         io.alt = 1;
         io.nsys = 2 * r.batch;  // system 2y + h: the parity-h rows of right-hand side y
     }

@@ -189,17 +189,27 @@ __device__ __forceinline__ void group_bar(int id, int nthreads)
 }
 
 // ---- Exact power-of-two renormalisation of a 2x2 matrix (keeps continuant
-// products in range without rounding).
+// products in range without rounding).  The factor 2^-e is assembled from the
+// exponent field e of the largest entry, so a renormalisation is a few integer
+// operations and one multiplication an entry; the factorisations run one per
+// row on their critical path.
+__device__ __forceinline__ double renorm_factor(double a, double b, double c, double d)
+{
+    const int h = max(max(__double2hiint(a) & 0x7fffffff, __double2hiint(b) & 0x7fffffff),
+                      max(__double2hiint(c) & 0x7fffffff, __double2hiint(d) & 0x7fffffff));
+    const int e = h >> 20;  // 0: zero or subnormal entries only; 2047: an infinity or NaN
+    return (e == 0 || e == 2047) ? 1.0 : __hiloint2double(max(2046 - e, 1) << 20, 0);
+}
 __device__ __forceinline__ void renorm2x2(double& a, double& b, double& c, double& d)
 {
-    double m = fmax(fmax(fabs(a), fabs(b)), fmax(fabs(c), fabs(d)));
-    if (m > 0.0 && isfinite(m)) {
-        int e = ilogb(m);
-        a = scalbn(a, -e);
-        b = scalbn(b, -e);
-        c = scalbn(c, -e);
-        d = scalbn(d, -e);
-    }
+    const double f = renorm_factor(a, b, c, d);
+    a *= f;
+    b *= f;
+    c *= f;
+    d *= f;
 }
+
+// floor(n / d) from the reciprocal fast_div_mul(d); exact for n d < 2^32.
+__device__ __forceinline__ unsigned fast_div(unsigned n, unsigned mul) { return mul ? __umulhi(n, mul) : n; }
 
 }  // namespace pfb

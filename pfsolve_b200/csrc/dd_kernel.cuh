@@ -66,14 +66,11 @@ __device__ __forceinline__ dd band_dd(const double* base, int64_t off, int64_t p
 
 __device__ __forceinline__ void renorm2x2_dd(dd& a, dd& b, dd& c, dd& d)
 {
-    double m = fmax(fmax(fabs(a.hi), fabs(b.hi)), fmax(fabs(c.hi), fabs(d.hi)));
-    if (m > 0.0 && isfinite(m)) {
-        const int e = ilogb(m);
-        a = dd(scalbn(a.hi, -e), scalbn(a.lo, -e));
-        b = dd(scalbn(b.hi, -e), scalbn(b.lo, -e));
-        c = dd(scalbn(c.hi, -e), scalbn(c.lo, -e));
-        d = dd(scalbn(d.hi, -e), scalbn(d.lo, -e));
-    }
+    const double f = renorm_factor(a.hi, b.hi, c.hi, d.hi);
+    a = dd(a.hi * f, a.lo * f);
+    b = dd(b.hi * f, b.lo * f);
+    c = dd(c.hi * f, c.lo * f);
+    d = dd(d.hi * f, d.lo * f);
 }
 
 // Exclusive scan of 2x2 double-double matrix products (row order).
@@ -101,14 +98,24 @@ __device__ __forceinline__ void group_matrix_scan_dd(GroupCtx& g, dd& a, dd& b, 
         }
         __syncwarp();
         group_bar(g.bar_id, g.nthr);
-        for (int w = 0; w < g.wg; ++w) {
-            const double* o = g.warp_area(w) + 16;
-            const dd oa = load_v<dd>(o), ob = load_v<dd>(o + 2), oc = load_v<dd>(o + 4), od = load_v<dd>(o + 6);
-            const dd na = dd_fma(oa, wa, ob * wc), nb = dd_fma(oa, wb, ob * wd);
-            const dd nc = dd_fma(oc, wa, od * wc), nd = dd_fma(oc, wb, od * wd);
-            wa = na; wb = nb; wc = nc; wd = nd;
-            renorm2x2_dd(wa, wb, wc, wd);
+        // the warps' products scanned over the lanes, as in group_matrix_scan
+        if (g.lane < g.W) {
+            const double* o = g.warp_area(g.lane) + 16;
+            wa = load_v<dd>(o); wb = load_v<dd>(o + 2); wc = load_v<dd>(o + 4); wd = load_v<dd>(o + 6);
         }
+        for (int s = 1; s < g.W; s <<= 1) {
+            const dd pa = O::shfl_up(wa, s), pb = O::shfl_up(wb, s), pc = O::shfl_up(wc, s), pd = O::shfl_up(wd, s);
+            if (g.lane >= s) {
+                const dd na = dd_fma(wa, pa, wb * pc), nb = dd_fma(wa, pb, wb * pd);
+                const dd nc = dd_fma(wc, pa, wd * pc), nd = dd_fma(wc, pb, wd * pd);
+                wa = na; wb = nb; wc = nc; wd = nd;
+                renorm2x2_dd(wa, wb, wc, wd);
+            }
+        }
+        const int src = g.wg > 0 ? g.wg - 1 : 0;
+        auto from = [&](dd v) { return dd(__shfl_sync(FULL, v.hi, src), __shfl_sync(FULL, v.lo, src)); };
+        wa = from(wa); wb = from(wb); wc = from(wc); wd = from(wd);
+        if (g.wg == 0) { wa = dd(1.0); wb = dd(0.0); wc = dd(0.0); wd = dd(1.0); }
         group_bar(g.bar_id, g.nthr);
     }
     a = dd_fma(ea, wa, eb * wc);
@@ -181,13 +188,13 @@ __device__ __forceinline__ void dd_prologue(const JwOperator& op, GroupCtx& g, i
             renorm2x2_dd(a, b, c, d);
         }
         group_matrix_scan_dd(g, a, b, c, d);
-        dd dprev = (s == 0) ? dd(1.0) : a / c;
+        dd mprev = (s == 0) ? dd(1.0) : c / a;  // reciprocal pivot of the row before
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             const int64_t i = s + j;
-            const dd dp = (i == 0) ? dd(1.0) : dd(1.0) - acs[j] / dprev;
+            const dd dp = (i == 0) ? dd(1.0) : dd_fma(-acs[j], mprev, dd(1.0));
             const dd dinv = dd(1.0) / dp;
-            dprev = dp;
+            mprev = dinv;
             const dd ai = (i >= 1 && i < M) ? bnd(op.off_sl, i) : dd(0.0);
             const dd ci = (i < M - 1) ? bnd(op.off_su, i) : dd(0.0);
             cf.l[j] = ai * dinv;
@@ -343,9 +350,8 @@ __global__ void __launch_bounds__(256) jw_dd_kernel(const JwOperator op, const J
 
 // The table, built by all NT threads of the CTA: thread tid takes rows
 // [tid Rp, tid Rp + Rp) of the group's T R rows (their pivots from a Moebius
-// scan over the CTA, as dd_prologue does over a group), then group 0 (tid <
-// T: one thread per chunk) forms the chunk products and the scans'
-// multipliers.  Same values as dd_prologue and chunk_solve compute per
+// scan over the CTA, as dd_prologue does over a group), then one thread per
+// chunk and direction forms the chunk products and the scans' multipliers.  Same values as dd_prologue and chunk_solve compute per
 // system, up to the association of the pivot products.
 template <class C>
 __device__ __noinline__ void dd_tbl_prologue(const JwOperator& op, dd* tab, dd* mul, double* scratch_all, int T,
@@ -367,7 +373,7 @@ __device__ __noinline__ void dd_tbl_prologue(const JwOperator& op, dd* tab, dd* 
     const int rows = T * R;
     const int Rp = (rows + NT - 1) / NT;
     const int64_t s = (int64_t)tid * Rp;
-    dd dprev(1.0);
+    dd mprev(1.0);  // reciprocal pivot of the row before
     if constexpr (C::kSV == SV_TRI) {
         dd a(1.0), b(0.0), c(0.0), d(1.0);
         for (int j = 0; j < Rp; ++j) {
@@ -382,7 +388,7 @@ __device__ __noinline__ void dd_tbl_prologue(const JwOperator& op, dd* tab, dd* 
             renorm2x2_dd(a, b, c, d);
         }
         group_matrix_scan_dd(gc, a, b, c, d);
-        dprev = (s == 0) ? dd(1.0) : a / c;
+        mprev = (s == 0) ? dd(1.0) : c / a;
     }
 #pragma unroll 1
     for (int j = 0; j < Rp; ++j) {
@@ -422,9 +428,9 @@ __device__ __noinline__ void dd_tbl_prologue(const JwOperator& op, dd* tab, dd* 
                 const dd ai = (i >= 1) ? bnd(op.off_sl, i) : dd(0.0);
                 const dd ci = (i < M - 1) ? bnd(op.off_su, i) : dd(0.0);
                 const dd ac = (i >= 1) ? ai * ((i - 1 < M - 1) ? bnd(op.off_su, i - 1) : dd(0.0)) : dd(0.0);
-                const dd dp = (i == 0) ? dd(1.0) : dd(1.0) - ac / dprev;
+                const dd dp = (i == 0) ? dd(1.0) : dd_fma(-ac, mprev, dd(1.0));
                 const dd dinv = dd(1.0) / dp;
-                dprev = dp;
+                mprev = dinv;
                 nl = -(ai * dinv);
                 nh = -(ci * dinv);
 #pragma unroll
@@ -441,38 +447,33 @@ __device__ __noinline__ void dd_tbl_prologue(const JwOperator& op, dd* tab, dd* 
         if constexpr (C::kBwd) at(C::P_NH, i) = nh;
     }
     __syncthreads();
-    if (tid >= T) return;
-    // group 0, thread t = tid: its chunk's products and the scans' multipliers
+    // one thread per chunk and direction: the chunk's products and the scans'
+    // multipliers (threads [0, T) -l, the next T -h where the CTA has them,
+    // else the same threads in turn)
     GroupCtx g = gc;
     g.W = T >> 5;
     g.nthr = T;
-    const int t = tid;
-    auto ch = [&](int p, int j) -> dd& { return tab[((size_t)p * R + j) * T + t]; };
-    if constexpr (C::kFwd) {
+    const bool both = NT >= 2 * T;
+    auto fill = [&](int t, int pn, int pp, int m0, bool up) {
+        auto ch = [&](int p, int j) -> dd& { return tab[((size_t)p * R + j) * T + t]; };
         dd p(1.0);
-#pragma unroll 1
-        for (int j = 0; j < R; ++j) {
-            p = ch(C::P_NL, j) * p;
-            ch(C::P_PL, j) = p;
+#pragma unroll 4
+        for (int k = 0; k < R; ++k) {
+            const int j = up ? k : R - 1 - k;
+            p = ch(pn, j) * p;
+            ch(pp, j) = p;
         }
-        const ScanMul<dd> m = scan_multipliers<dd, true>(g, p);
+        const ScanMul<dd> m = up ? scan_multipliers<dd, true>(g, p) : scan_multipliers<dd, false>(g, p);
 #pragma unroll
-        for (int k = 0; k < 5; ++k) mul[k * T + t] = m.lev[k];
-        mul[5 * T + t] = m.Ae;
-        mul[6 * T + t] = m.Aw;
-    }
+        for (int k = 0; k < 5; ++k) mul[(m0 + k) * T + t] = m.lev[k];
+        mul[(m0 + 5) * T + t] = m.Ae;
+        mul[(m0 + 6) * T + t] = m.Aw;
+    };
+    if constexpr (C::kFwd)
+        if (tid < T) fill(tid, C::P_NL, C::P_PL, 0, true);
     if constexpr (C::kBwd) {
-        dd p(1.0);
-#pragma unroll 1
-        for (int j = R - 1; j >= 0; --j) {
-            p = ch(C::P_NH, j) * p;
-            ch(C::P_PH, j) = p;
-        }
-        const ScanMul<dd> m = scan_multipliers<dd, false>(g, p);
-#pragma unroll
-        for (int k = 0; k < 5; ++k) mul[(C::kMul + k) * T + t] = m.lev[k];
-        mul[(C::kMul + 5) * T + t] = m.Ae;
-        mul[(C::kMul + 6) * T + t] = m.Aw;
+        const int t = both ? tid - T : tid;
+        if (t >= 0 && t < T) fill(t, C::P_NH, C::P_PH, C::kMul, false);
     }
 }
 

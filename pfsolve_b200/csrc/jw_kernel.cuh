@@ -100,23 +100,30 @@ __host__ size_t jw_smem_bytes(int W, int G)
 
 // Storage position of row i in the reference's band order (reorder_i0,
 // pfSolve_Plan_JonesWorland.h:66-142): register-major within each piece of
-// perm_piece rows (the whole system when perm_piece == 0).
+// perm_piece rows (the whole system when perm_piece == 0).  Every table build
+// calls it several times a row: the divisions are 32-bit multiplications by
+// host-made reciprocals (as 64-bit divisions they were most of the 12 us that
+// a tridiagonal table at N = 512 added to a launch).
 __device__ __forceinline__ int64_t band_pos(const JwOperator& op, int64_t i)
 {
-    if (op.alt) return (i % op.alt_R) * op.alt_T + op.alt_h * (op.alt_T >> 1) + i / op.alt_R;
+    const int row = (int)i;
+    if (op.alt) {
+        const int e = (int)fast_div((unsigned)row, op.alt_mul);
+        return (int64_t)(row - e * (int)op.alt_R) * op.alt_T + op.alt_h * (op.alt_T >> 1) + e;
+    }
     if (!op.perm) return i;
-    int64_t base = 0, li = i, m = op.perm_m, ce = op.perm_ceil, fl = op.perm_floor;
+    int base = 0, li = row, m = (int)op.perm_m, ce = (int)op.perm_ceil, fl = (int)op.perm_floor;
     if (op.perm_piece) {
-        const int64_t piece = i / op.perm_piece;
-        base = piece * op.perm_piece;
-        li = i - base;
-        if (base + op.perm_piece > op.M) {
-            m = op.perm_lm;
-            ce = op.perm_lceil;
-            fl = op.perm_lfloor;
+        const int size = (int)op.perm_piece;
+        base = (int)fast_div((unsigned)row, op.piece_mul) * size;
+        li = row - base;
+        if (base + size > (int)op.M) {
+            m = (int)op.perm_lm;
+            ce = (int)op.perm_lceil;
+            fl = (int)op.perm_lfloor;
         }
     }
-    const int64_t t = li / op.perm_r, j = li - t * op.perm_r;
+    const int t = (int)fast_div((unsigned)li, op.perm_mul), j = li - t * (int)op.perm_r;
     return base + t + ((j < m) ? j * ce : m * ce + (j - m) * fl);
 }
 
@@ -435,13 +442,27 @@ __device__ __forceinline__ void group_matrix_scan(GroupCtx& g, double& a, double
         if (g.lane == 31) { my[0] = a; my[1] = b; my[2] = c; my[3] = d; }
         __syncwarp();
         group_bar(g.bar_id, g.nthr);
-        for (int w = 0; w < g.wg; ++w) {
-            const double* o = g.warp_area(w) + 24;
-            double na = o[0] * wa + o[1] * wc, nb = o[0] * wb + o[1] * wd;
-            double nc = o[2] * wa + o[3] * wc, nd = o[2] * wb + o[3] * wd;
-            wa = na; wb = nb; wc = nc; wd = nd;
-            renorm2x2(wa, wb, wc, wd);
+        // every warp scans the warps' products over its lanes (log2 W levels
+        // instead of a chain of up to W - 1 products) and takes the one
+        // before its own
+        if (g.lane < g.W) {
+            const double* o = g.warp_area(g.lane) + 24;
+            wa = o[0]; wb = o[1]; wc = o[2]; wd = o[3];
         }
+        for (int s = 1; s < g.W; s <<= 1) {
+            const double pa = __shfl_up_sync(FULL, wa, s), pb = __shfl_up_sync(FULL, wb, s);
+            const double pc = __shfl_up_sync(FULL, wc, s), pd = __shfl_up_sync(FULL, wd, s);
+            if (g.lane >= s) {
+                const double na = wa * pa + wb * pc, nb = wa * pb + wb * pd;
+                const double nc = wc * pa + wd * pc, nd = wc * pb + wd * pd;
+                wa = na; wb = nb; wc = nc; wd = nd;
+                renorm2x2(wa, wb, wc, wd);
+            }
+        }
+        const int src = g.wg > 0 ? g.wg - 1 : 0;
+        wa = __shfl_sync(FULL, wa, src); wb = __shfl_sync(FULL, wb, src);
+        wc = __shfl_sync(FULL, wc, src); wd = __shfl_sync(FULL, wd, src);
+        if (g.wg == 0) { wa = 1; wb = 0; wc = 0; wd = 1; }
         group_bar(g.bar_id, g.nthr);
     }
     a = ea * wa + eb * wc;
@@ -467,19 +488,23 @@ __device__ __forceinline__ void jw_row_weights(const JwOperator& op, int64_t i, 
         w[KL] = vd;
         if constexpr (NB - KL - 1 >= 1) w[KL + 1] = vu;
     } else {
+        // row i + pv of A meets the weight at column i + k as its band entry
+        // kk = k - pv; unrolled, so that a row's loads are issued together
         const int kla = op.dg_lda - 1 - op.dg_ku;
+#pragma unroll
         for (int pv = -1; pv <= 1; ++pv) {
             const double vp = (pv < 0) ? vl : (pv == 0 ? vd : vu);
             const int64_t p = i + pv;
-            if (vp == 0.0 || p < 0 || p >= M) continue;
-            for (int kk = -kla; kk <= op.dg_ku; ++kk) {
-                const int64_t c = p + kk;
-                if (c < 0 || c >= M || ((op.dg_skip >> (op.dg_ku - kk)) & 1)) continue;
-                const double a = band_at(op, op.dgbmv, op.dg_off + (int64_t)(op.dg_ku - kk) * M + c);
-                const int64_t k = c - i;  // within [-KL, KU] by construction of the plan
+            // (not on vp's value: that would hold the loads below until it arrives)
+            const bool pok = (pv == 0 || op.mvj == (pv < 0 ? MVJ_LOWER : MVJ_UPPER)) && p >= 0 && p < M;
 #pragma unroll
-                for (int q = 0; q < NB; ++q)
-                    if (q - KL == (int)k) w[q] = __fma_rn(vp, a, w[q]);
+            for (int q = 0; q < NB; ++q) {
+                const int kk = q - KL - pv;
+                const int64_t c = i + (q - KL);
+                const bool ok = pok && kk >= -kla && kk <= op.dg_ku && c >= 0 && c < M &&
+                                !((op.dg_skip >> ((op.dg_ku - kk) & 63)) & 1);
+                const double a = ok ? band_at(op, op.dgbmv, op.dg_off + (int64_t)(op.dg_ku - kk) * M + c) : 0.0;
+                if (ok && vp != 0.0) w[q] = __fma_rn(vp, a, w[q]);
             }
         }
     }
@@ -519,33 +544,30 @@ __device__ __forceinline__ void jw_prologue(const JwOperator& op, GroupCtx& g, i
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             const int64_t i = s + j;
-            double ac = 0.0;
-            if (i >= 1 && i < M) {
-                const double ai = band(op, op.off_sl, i);
-                const double cim1 = (i - 1 < M - 1) ? band(op, op.off_su, i - 1) : 0.0;
-                ac = ai * cim1;
-            }
+            a64[j] = (i >= 1 && i < M) ? band(op, op.off_sl, i) : 0.0;
+            c64[j] = (i < M - 1) ? band(op, op.off_su, i) : 0.0;
+        }
+        const double cprev = (s >= 1 && s < M) ? band(op, op.off_su, s - 1) : 0.0;
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const double ac = a64[j] * (j ? c64[j - 1] : cprev);
             acs[j] = ac;
             const double na = a - ac * c, nb = b - ac * d;
             c = a; d = b; a = na; b = nb;
             renorm2x2(a, b, c, d);
         }
         group_matrix_scan(g, a, b, c, d);
-        // incoming vector = Q * (1, 0)^T = (a, c): d'_{s-1} = a / c
-        double dprev = (s == 0) ? 1.0 : a / c;
+        // incoming vector = Q * (1, 0)^T = (a, c): 1 / d'_{s-1} = c / a
+        double mprev = (s == 0) ? 1.0 : c / a;
 #pragma unroll
         for (int j = 0; j < R; ++j) {
             const int64_t i = s + j;
-            const double dp = (i == 0) ? 1.0 : 1.0 - acs[j] / dprev;
-            const double dinv = 1.0 / dp;
-            dprev = dp;
-            const double ai = (i >= 1 && i < M) ? band(op, op.off_sl, i) : 0.0;
-            const double ci = (i < M - 1) ? band(op, op.off_su, i) : 0.0;
-            l64[j] = ai * dinv;
-            h64[j] = ci * dinv;
+            const double dp = (i == 0) ? 1.0 : __fma_rn(-acs[j], mprev, 1.0);
+            const double dinv = 1.0 / dp;  // one division a row
+            mprev = dinv;
+            l64[j] = a64[j] * dinv;
+            h64[j] = c64[j] * dinv;
             m64[j] = dinv;
-            a64[j] = ai;
-            c64[j] = ci;
         }
     } else if constexpr (C::kSV == SV_LOWER) {
 #pragma unroll

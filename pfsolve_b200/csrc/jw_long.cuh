@@ -143,26 +143,31 @@ __device__ void lg_prologue(const JwOperator& op, double* table, double* scratch
     g.bar_id = 1;
     g.seq = 0;
     g.scratch = scratch;
-    auto mstep = [&](int64_t i, double& a, double& b, double& cc, double& d) {
-        double ac = 0.0;
-        if (i >= 1 && i < M) ac = band(op, op.off_sl, i) * band(op, op.off_su, i - 1);
-        const double na = a - ac * cc, nb = b - ac * d;
-        cc = a;
-        d = b;
-        a = na;
-        b = nb;
-        renorm2x2(a, b, cc, d);
-    };
-    double dprev = 1.0;
+    double mprev = 1.0;  // reciprocal pivot of the row before
     const int Rp = (S + nthr - 1) / nthr;
     const int64_t s = s0 + (int64_t)tid * Rp;
     if constexpr (C::SV == SV_TRI) {
         // this thread's rows of the slice, then the product of the slice's
         // preceding chunks
         double a = 1, b = 0, cc = 0, d = 1;
-        for (int j = 0; j < Rp; ++j) {
-            const int64_t i = s + j;
-            if (i < s0 + S) mstep(i, a, b, cc, d);
+        for (int j0 = 0; j0 < Rp; j0 += 4) {  // loads in blocks of 4 ahead of their chain
+            double ac[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int64_t i = s + j0 + e;
+                const bool ok = j0 + e < Rp && i < s0 + S && i >= 1 && i < M;
+                ac[e] = ok ? band(op, op.off_sl, i) * band(op, op.off_su, i - 1) : 0.0;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (j0 + e >= Rp || s + j0 + e >= s0 + S) break;
+                const double na = a - ac[e] * cc, nb = b - ac[e] * d;
+                cc = a;
+                d = b;
+                a = na;
+                b = nb;
+                renorm2x2(a, b, cc, d);
+            }
         }
         const double pa = a, pb = b, pc = cc, pd = d;
         group_matrix_scan(g, a, b, cc, d);
@@ -204,8 +209,9 @@ __device__ void lg_prologue(const JwOperator& op, double* table, double* scratch
         (void)q4;
         // full prefix = (slice prefix) * Q; incoming vector = prefix * (1, 0)^T
         const double fa = a * qa + b * qc, fc = cc * qa + d * qc;
-        dprev = (s == 0) ? 1.0 : fa / fc;
+        mprev = (s == 0) ? 1.0 : fc / fa;
     }
+#pragma unroll 2
     for (int j = 0; j < Rp; ++j) {
         const int64_t li = (int64_t)tid * Rp + j;  // row within the slice
         if (li >= S) break;
@@ -219,9 +225,9 @@ __device__ void lg_prologue(const JwOperator& op, double* table, double* scratch
                 const double ai = (i >= 1) ? band(op, op.off_sl, i) : 0.0;
                 const double ci = (i < M - 1) ? band(op, op.off_su, i) : 0.0;
                 const double ac = (i >= 1) ? ai * band(op, op.off_su, i - 1) : 0.0;
-                const double dp = (i == 0) ? 1.0 : 1.0 - ac / dprev;
-                m = 1.0 / dp;
-                dprev = dp;
+                const double dp = (i == 0) ? 1.0 : __fma_rn(-ac, mprev, 1.0);
+                m = 1.0 / dp;  // one division a row
+                mprev = m;
                 nl = -(ai * m);
                 nh = -(ci * m);
             } else if constexpr (C::SV == SV_LOWER) {

@@ -236,6 +236,12 @@ __device__ __forceinline__ int swz_row(int t)
 }
 
 // ---- Coefficient table, built once per CTA by all of its threads.
+// It stands between a launch and its first solve (the first systems' copies
+// are in flight meanwhile), and small batches pay little else, so it is kept
+// short: the bands' loads in blocks ahead of the dependent chains, one division
+// a pivot, cheap band positions and renormalisations, and a logarithmic scan
+// over the warps.  A tridiagonal launch of 8 systems took 16.7 us at N = 512,
+// 26.5 at 2 048 and 87.9 at 4 096 before that, and takes 8.5, 13.7 and 45.3.
 // Plane p, row i = R*tt + j (tt: thread of a group) is the double at
 // [((p*U + j/2)*T + tt)*2 + (j&1)]: thread tt reads rows 2u, 2u+1 of a plane
 // as one 16-byte word, lanes on consecutive words.
@@ -248,95 +254,117 @@ __device__ void st_prologue_system(const JwOperator& op, int h, typename C::CT* 
     const int nthr = blockDim.x, tid = threadIdx.x;
     const int Rp = (rows + nthr - 1) / nthr;
     const int64_t s = (int64_t)tid * Rp;
-    double dprev = 1.0;
+    // Rows in blocks of PB, each block's band loads issued together ahead of
+    // its dependent chain.
+    constexpr int PB = NB == 1 ? 4 : 2;
+    double mprev = 1.0;  // reciprocal pivot of the row before
     if constexpr (C::SV == SV_TRI) {
         // Moebius product of this thread's rows, then the CTA-wide scan gives
         // the pivot entering them (same recurrence as jw_prologue).
         double a = 1, b = 0, c = 0, d = 1;
-        for (int j = 0; j < Rp; ++j) {
-            const int64_t i = s + j;
-            double ac = 0.0;
-            if (i >= 1 && i < M) ac = band(op, op.off_sl, i) * band(op, op.off_su, i - 1);
-            const double na = a - ac * c, nb = b - ac * d;
-            c = a;
-            d = b;
-            a = na;
-            b = nb;
-            renorm2x2(a, b, c, d);
+        for (int j0 = 0; j0 < Rp; j0 += 4) {
+            double ac[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const int64_t i = s + j0 + e;
+                const bool ok = j0 + e < Rp && i >= 1 && i < M;
+                ac[e] = ok ? band(op, op.off_sl, i) * band(op, op.off_su, i - 1) : 0.0;
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (j0 + e >= Rp) break;
+                const double na = a - ac[e] * c, nb = b - ac[e] * d;
+                c = a;
+                d = b;
+                a = na;
+                b = nb;
+                renorm2x2(a, b, c, d);
+            }
         }
         group_matrix_scan(g, a, b, c, d);
-        dprev = (s == 0) ? 1.0 : a / c;
+        mprev = (s == 0) ? 1.0 : c / a;
     }
-    for (int j = 0; j < Rp; ++j) {
-        const int64_t i = s + j;
-        if (i >= rows) break;
-        double w[NB];
-        double nl = 0.0, nh = 0.0, sc = 0.0, m = 1.0, al = 0.0, cu = 0.0;
-        if (i < M) {
-            jw_row_weights<C::KL, NB>(op, i, w);
-            if constexpr (C::SV == SV_TRI) {
-                const double ai = (i >= 1) ? band(op, op.off_sl, i) : 0.0;
-                const double ci = (i < M - 1) ? band(op, op.off_su, i) : 0.0;
-                const double ac = (i >= 1) ? ai * band(op, op.off_su, i - 1) : 0.0;
-                const double dp = (i == 0) ? 1.0 : 1.0 - ac / dprev;
-                m = 1.0 / dp;
-                dprev = dp;
-                nl = -(ai * m);
-                nh = -(ci * m);
-                al = ai;
-                cu = ci;
-            } else if constexpr (C::SV == SV_LOWER) {
-                al = (i >= 1) ? band(op, op.off_sl, i) : 0.0;
-                nl = -al;
-            } else if constexpr (C::SV == SV_UPPER) {
-                cu = (i < M - 1) ? band(op, op.off_su, i) : 0.0;
-                nh = -cu;
-            }
-            if constexpr (!C::MIXED) {
+    for (int j0 = 0; j0 < Rp; j0 += PB) {
+        double wr[PB][NB], al_[PB], cu_[PB], ac_[PB];
 #pragma unroll
-                for (int k = 0; k < NB; ++k) w[k] *= m;
-            }
-            if constexpr (C::SCALE) sc = scale_factor(op.scale_kind, i, op.lshift, op.scale_s);
-        } else {
+        for (int e = 0; e < PB; ++e) {
+            const int64_t i = s + j0 + e;
+            al_[e] = cu_[e] = ac_[e] = 0.0;
 #pragma unroll
-            for (int k = 0; k < NB; ++k) w[k] = 0.0;
+            for (int k = 0; k < NB; ++k) wr[e][k] = 0.0;
+            if (j0 + e < Rp && i < M) {
+                jw_row_weights<C::KL, NB>(op, i, wr[e]);
+                if constexpr (C::SV == SV_TRI || C::SV == SV_LOWER)
+                    if (i >= 1) al_[e] = band(op, op.off_sl, i);
+                if constexpr (C::SV == SV_TRI || C::SV == SV_UPPER)
+                    if (i < M - 1) cu_[e] = band(op, op.off_su, i);
+                if constexpr (C::SV == SV_TRI)
+                    if (i >= 1) ac_[e] = band(op, op.off_su, i - 1);
+            }
         }
-        const int64_t si = C::S * i + h;  // staged row
-        const int tt = (int)(si / R), jj = (int)(si % R);
-        auto put = [&](int p, double v) {
-            table[(((size_t)p * U + (jj >> 1)) * C::TP + tt) * 2 + (jj & 1)] = (typename C::CT)v;
-        };
-        if constexpr (C::QUAD) {  // float4 per (row quad, thread)
-            const int q4 = jj >> 2, e4 = jj & 3;
-            auto putq = [&](int p, double v) {
-                reinterpret_cast<float*>(table)[(((size_t)p * C::U4 + q4) * C::TP + tt) * 4 + e4] = (float)v;
+#pragma unroll
+        for (int e = 0; e < PB; ++e) {
+            const int64_t i = s + j0 + e;
+            if (j0 + e >= Rp || i >= rows) break;
+            double (&w)[NB] = wr[e];
+            const double al = al_[e], cu = cu_[e];
+            double nl = 0.0, nh = 0.0, sc = 0.0, m = 1.0;
+            if (i < M) {
+                if constexpr (C::SV == SV_TRI) {
+                    // pivot d_i = 1 - a_i c_{i-1} / d_{i-1}, one division a row
+                    const double dp = (i == 0) ? 1.0 : __fma_rn(-(al * ac_[e]), mprev, 1.0);
+                    m = 1.0 / dp;
+                    mprev = m;
+                    nl = -(al * m);
+                    nh = -(cu * m);
+                } else if constexpr (C::SV == SV_LOWER) {
+                    nl = -al;
+                } else if constexpr (C::SV == SV_UPPER) {
+                    nh = -cu;
+                }
+                if constexpr (!C::MIXED) {
+#pragma unroll
+                    for (int k = 0; k < NB; ++k) w[k] *= m;
+                }
+                if constexpr (C::SCALE) sc = scale_factor(op.scale_kind, i, op.lshift, op.scale_s);
+            }
+            const int64_t si = C::S * i + h;  // staged row
+            const int tt = (int)(si / R), jj = (int)(si % R);
+            auto put = [&](int p, double v) {
+                table[(((size_t)p * U + (jj >> 1)) * C::TP + tt) * 2 + (jj & 1)] = (typename C::CT)v;
+            };
+            if constexpr (C::QUAD) {  // float4 per (row quad, thread)
+                const int q4 = jj >> 2, e4 = jj & 3;
+                auto putq = [&](int p, double v) {
+                    reinterpret_cast<float*>(table)[(((size_t)p * C::U4 + q4) * C::TP + tt) * 4 + e4] = (float)v;
+                };
+#pragma unroll
+                for (int k = 0; k < NB; ++k) putq(k, w[k]);
+                if constexpr (C::FWD) putq(C::P_NL, nl);
+                if constexpr (C::BWD) putq(C::P_NH, nh);
+                if constexpr (C::SCALE) putq(C::P_SC, sc);
+                continue;
+            }
+            auto put32 = [&](int p, int k, double v) {
+                reinterpret_cast<float*>(table)[(((size_t)p * U + (jj >> 1)) * C::TP + tt) * 4 + k + (jj & 1)] = (float)v;
             };
 #pragma unroll
-            for (int k = 0; k < NB; ++k) putq(k, w[k]);
-            if constexpr (C::FWD) putq(C::P_NL, nl);
-            if constexpr (C::BWD) putq(C::P_NH, nh);
-            if constexpr (C::SCALE) putq(C::P_SC, sc);
-            continue;
-        }
-        auto put32 = [&](int p, int k, double v) {
-            reinterpret_cast<float*>(table)[(((size_t)p * U + (jj >> 1)) * C::TP + tt) * 4 + k + (jj & 1)] = (float)v;
-        };
-#pragma unroll
-        for (int k = 0; k < NB; ++k) put(k, w[k]);
-        if constexpr (C::MIXED) {
-            if constexpr (C::FWD) put(C::P_AL, al);
-            if constexpr (C::BWD) put(C::P_CU, cu);
-            put32(C::P_F1, 0, m);
-            put32(C::P_F1, 2, nl);
-            if constexpr (C::BWD) {
-                put32(C::P_F2, 0, nh);
-                put32(C::P_F2, 2, 0.0);
+            for (int k = 0; k < NB; ++k) put(k, w[k]);
+            if constexpr (C::MIXED) {
+                if constexpr (C::FWD) put(C::P_AL, al);
+                if constexpr (C::BWD) put(C::P_CU, cu);
+                put32(C::P_F1, 0, m);
+                put32(C::P_F1, 2, nl);
+                if constexpr (C::BWD) {
+                    put32(C::P_F2, 0, nh);
+                    put32(C::P_F2, 2, 0.0);
+                }
+            } else {
+                if constexpr (C::FWD) put(C::P_NL, nl);
+                if constexpr (C::BWD) put(C::P_NH, nh);
             }
-        } else {
-            if constexpr (C::FWD) put(C::P_NL, nl);
-            if constexpr (C::BWD) put(C::P_NH, nh);
+            if constexpr (C::SCALE) put(C::P_SC, sc);
         }
-        if constexpr (C::SCALE) put(C::P_SC, sc);
     }
 }
 
@@ -356,51 +384,39 @@ __device__ void st_prologue(const JwOperator& op, typename C::CT* table, double*
     g.scratch = scratch_all;
     if constexpr (!C::ALT) {
         st_prologue_system<C>(op, 0, table, g);
-        if constexpr (C::PROD && (C::FWD || C::BWD)) {
-            // one thread per chunk: the products of -l up to each row and of
-            // -h from each row on, in the order the solve used to form them
+        if constexpr (C::PRODS && (C::FWD || C::BWD)) {
+            // one thread per chunk and direction: the products of -l up to
+            // each row and of -h from each row on, in the order the solve
+            // used to form them; a chunk's factors are loaded together ahead
+            // of the chain
             __syncthreads();
-            auto at = [&](int p, int j, int tt) -> double& {
-                return table[(((size_t)p * C::U + (j >> 1)) * C::TP + tt) * 2 + (j & 1)];
+            using CT = typename C::CT;
+            auto at = [&](int p, int j, int tt) -> CT& {
+                if constexpr (C::QUAD) return table[(((size_t)p * C::U4 + (j >> 2)) * C::TP + tt) * 4 + (j & 3)];
+                else return table[(((size_t)p * C::U + (j >> 1)) * C::TP + tt) * 2 + (j & 1)];
             };
-            for (int tt = threadIdx.x; tt < C::T; tt += blockDim.x) {
-                if constexpr (C::FWD) {
-                    double pr = 1.0;
-                    for (int j = 0; j < C::R; ++j) {
-                        pr = at(C::P_NL, j, tt) * pr;
-                        at(C::P_PL, j, tt) = pr;
+            for (int k = threadIdx.x; k < 2 * C::T; k += blockDim.x) {
+                const bool up = k < C::T;  // whole warps
+                const int tt = up ? k : k - C::T;
+                if (up ? !C::FWD : !C::BWD) continue;
+                CT v[C::R];
+                if (up) {
+                    if constexpr (C::FWD) {
+#pragma unroll
+                        for (int j = 0; j < C::R; ++j) v[j] = at(C::P_NL, j, tt);
+#pragma unroll
+                        for (int j = 1; j < C::R; ++j) v[j] = v[j] * v[j - 1];
+#pragma unroll
+                        for (int j = 0; j < C::R; ++j) at(C::P_PL, j, tt) = v[j];
                     }
-                }
-                if constexpr (C::BWD) {
-                    double pr = 1.0;
-                    for (int j = C::R - 1; j >= 0; --j) {
-                        pr = at(C::P_NH, j, tt) * pr;
-                        at(C::P_PH, j, tt) = pr;
-                    }
-                }
-            }
-        }
-        if constexpr (C::QUAD && (C::FWD || C::BWD)) {
-            // one thread per chunk: the products of -l up to each row and of
-            // -h from each row on, in the order the solve used to form them
-            __syncthreads();
-            float* tf = reinterpret_cast<float*>(table);
-            auto at = [&](int p, int j, int tt) -> float& {
-                return tf[(((size_t)p * C::U4 + (j >> 2)) * C::TP + tt) * 4 + (j & 3)];
-            };
-            for (int tt = threadIdx.x; tt < C::T; tt += blockDim.x) {
-                if constexpr (C::FWD) {
-                    float pr = 1.0f;
-                    for (int j = 0; j < C::R; ++j) {
-                        pr = at(C::P_NL, j, tt) * pr;
-                        at(C::P_PL, j, tt) = pr;
-                    }
-                }
-                if constexpr (C::BWD) {
-                    float pr = 1.0f;
-                    for (int j = C::R - 1; j >= 0; --j) {
-                        pr = at(C::P_NH, j, tt) * pr;
-                        at(C::P_PH, j, tt) = pr;
+                } else {
+                    if constexpr (C::BWD) {
+#pragma unroll
+                        for (int j = 0; j < C::R; ++j) v[j] = at(C::P_NH, j, tt);
+#pragma unroll
+                        for (int j = C::R - 2; j >= 0; --j) v[j] = v[j] * v[j + 1];
+#pragma unroll
+                        for (int j = 0; j < C::R; ++j) at(C::P_PH, j, tt) = v[j];
                     }
                 }
             }

@@ -16,6 +16,10 @@ enum : int { PREC_F64 = 0, PREC_MIXED = 1, PREC_DD = 2, PREC_DD_F64MEM = 3, PREC
 // Precisions whose buffers (bands, dgbmv matrix, right-hand sides) hold FP32 values.
 constexpr bool prec_f32_storage(int prec) { return prec == PREC_F32 || prec == PREC_F64_F32MEM; }
 
+// Reciprocal ceil(2^32 / d) of a divisor d >= 1 for fast_div (0 for d = 1).
+// Rows (< 2^16) over rows a lane (<= 68) or rows a piece (256): n d < 2^32.
+inline unsigned fast_div_mul(int64_t d) { return d > 1 ? (unsigned)(((1ull << 32) + (uint64_t)d - 1) / (uint64_t)d) : 0u; }
+
 // The matrix side of a JW step: where the bands live and how to read them.
 struct JwOperator {
     const double* bands;  // JW band buffer (FP64, or FP32 values when bands32)
@@ -27,6 +31,7 @@ struct JwOperator {
     // and the ceil / floor row counts; the partial last piece has its own
     int64_t perm_r, perm_m, perm_ceil, perm_floor;
     int64_t perm_piece, perm_lm, perm_lceil, perm_lfloor;
+    unsigned perm_mul, piece_mul;  // reciprocals of perm_r and perm_piece (fast_div)
     const double* dgbmv;  // fused general band matrix (band-major), or nullptr
     int64_t dg_off;
     int dg_lda, dg_ku;
@@ -41,6 +46,7 @@ struct JwOperator {
     // rows (entry of row r = 2 e + h at (e % alt_R) alt_T + h alt_T/2 + e / alt_R)
     int alt, alt_h;
     int64_t alt_T, alt_R;
+    unsigned alt_mul;  // reciprocal of alt_R (fast_div)
     int bands32;  // bands and the dgbmv matrix hold FP32 values (FP32-storage precisions)
 };
 

@@ -58,6 +58,8 @@ inline void set_band_order(int64_t M, JwOperator& op)
     op.perm_ceil = (full + r - 1) / r;
     op.perm_floor = full / r;
     const int64_t last = piece ? (M % piece) : 0;
+    op.perm_mul = fast_div_mul(r);
+    op.piece_mul = fast_div_mul(piece);
     op.perm_lm = last % r;
     op.perm_lceil = (last + r - 1) / r;
     op.perm_lfloor = last / r;
