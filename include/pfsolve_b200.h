@@ -507,7 +507,8 @@ PFSOLVE_API uint64_t PfSolveStreamingLaunchCount(void);
 enum {
     PFSOLVE_KERNEL_NONE = 0,      /* no launch yet on this thread */
     PFSOLVE_KERNEL_GROUP = 1,     /* jw_step_kernel: a group of warps per system, cp.async staging */
-    PFSOLVE_KERNEL_STREAMING = 2, /* jw_stream_kernel: whole systems staged by TMA */
+    PFSOLVE_KERNEL_STREAMING = 2, /* jw_stream_kernel: whole systems staged by TMA, or by element copies where
+                                     no tensor map describes the rows (odd strides, offsets or row counts) */
     PFSOLVE_KERNEL_LONG = 3,      /* jw_long_kernel: long systems in two passes over slices */
     PFSOLVE_KERNEL_CLUSTER = 4,   /* jw_cluster_kernel: one thread-block cluster per long system */
     PFSOLVE_KERNEL_STEPS = 5,     /* jw_steps_kernel: K consecutive steps */

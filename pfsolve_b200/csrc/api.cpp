@@ -47,6 +47,10 @@ struct AppState {
     // streaming variant (FP64, TMA-staged systems), used when a launch's
     // buffers allow it; `variant` serves the other launches
     const StreamVariant* stream_v = nullptr;
+    // the streaming kernel with element copies, for launches whose rows no
+    // tensor map describes
+    const StreamVariant* elem_v = nullptr;
+    int elem_G = 0, elem_max_blocks = 0, elem_nbuf = 2;
     int stream_G = 0, stream_max_blocks = 0;
     int stream_nbuf = 2;  // staging buffers per group
     int nbuf_req = 0;     // caller's staging buffers per group (0: choose)
@@ -92,6 +96,8 @@ struct AppState {
         int R, W, G, max_blocks;
         const StreamVariant* stream_v;
         int stream_G, stream_max_blocks, stream_nbuf;
+        const StreamVariant* elem_v;
+        int elem_G, elem_max_blocks, elem_nbuf;
     };
     std::vector<ChainPlan> chain_plans;
     // streams
@@ -157,6 +163,60 @@ int pick_rows_per_thread(int64_t M, int requested)
     return 16;
 }
 
+// Groups per CTA and staging buffers per group of a streaming variant: the
+// most groups that fit shared memory, two staging buffers per group -- three
+// for FP32 storage and arithmetic where they fit beside as many groups -- (a
+// caller's request: the most groups that fit with it).  Measured at
+// N = 512 (131 072 systems): 3 or 4 buffers per group were no faster
+// for FP64, the mixed mode or FP64 arithmetic on FP32 storage, 3 %
+// faster for FP32 (its 2-KB systems, solved fastest, need more of them
+// in flight), and where they cost groups (the config-2 chain) much
+// slower.
+bool stream_groups(AppState* s, const StreamVariant* v, int* G_out, int* nbuf_out, int* max_blocks)
+{
+    const int T = 32 * v->W;
+    auto fits = [&](int G, int nb, int* blocks) {
+        const size_t smem = v->smem_bytes(G, nb);
+        if (smem > 227 * 1024 || !allow_max_smem(v->func)) return false;
+        return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, v->func, v->threads(G), smem) == cudaSuccess &&
+               *blocks >= 1;
+    };
+    const bool req = s->nbuf_req >= 2 && s->nbuf_req <= kStMaxBuffers;
+    for (int G = std::min(v->max_threads / T, 15); G >= 1; --G) {
+        int blocks = 0;
+        int nb = req ? s->nbuf_req : 2;
+        if (!req && s->prec == PREC_F32 && fits(G, 3, &blocks)) nb = 3;
+        if (!fits(G, nb, &blocks)) continue;
+        *G_out = G;
+        *nbuf_out = nb;
+        *max_blocks = blocks * s->num_sms;
+        return true;
+    }
+    return false;
+}
+
+// The streaming kernel with element copies for a plan that has a group-kernel
+// variant: launches whose rows no tensor map describes (odd strides or
+// offsets, row counts that the rows per thread do not divide) take it instead
+// of the group kernel.  The shortest compiled capacity that holds M rows: 4,
+// 8, then 16 rows per thread of one warp, 16 of two and four warps, 32 of four.
+void choose_elem(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
+{
+    s->elem_v = nullptr;
+    if ((s->prec != PREC_F64 && s->prec != PREC_MIXED && !prec_f32_storage(s->prec)) || s->no_stream || s->alt) return;
+    static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 2}, {32, 4}};
+    for (const auto& rw : shapes) {
+        if (32 * (int64_t)rw[0] * rw[1] < M || (s->R_req && rw[0] != s->R_req)) continue;
+        const StreamVariant* v =
+            find_stream_variant(rw[0], rw[1], s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, 0, 1);
+        if (v && stream_groups(s, v, &s->elem_G, &s->elem_nbuf, &s->elem_max_blocks)) {
+            s->elem_v = v;
+            break;
+        }
+    }
+    cudaGetLastError();
+}
+
 // Streaming variant for M rows: rows per thread R (the caller's choice, else
 // the compiled R whose groups leave the fewest idle rows, 16 first), W warps
 // per system, and the most groups per CTA that fit shared memory.  ALT: M
@@ -187,31 +247,8 @@ bool choose_stream(AppState* s, int64_t M, int LIN, int LOUT, int SCALE, bool al
         const StreamVariant* v =
             find_stream_variant(cand[i][0], cand[i][1], s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, alt);
         if (!v) continue;
-        const int T = 32 * v->W;
-        // Most groups first, two staging buffers per group -- three for FP32
-        // storage and arithmetic where they fit beside as many groups -- (a
-        // caller's request: the most groups that fit with it).  Measured at
-        // N = 512 (131 072 systems): 3 or 4 buffers per group were no faster
-        // for FP64, the mixed mode or FP64 arithmetic on FP32 storage, 3 %
-        // faster for FP32 (its 2-KB systems, solved fastest, need more of them
-        // in flight), and where they cost groups (the config-2 chain) much
-        // slower.
-        auto fits = [&](int G, int nb, int* blocks) {
-            const size_t smem = v->smem_bytes(G, nb);
-            if (smem > 227 * 1024 || !allow_max_smem(v->func)) return false;
-            return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, v->func, T * G, smem) == cudaSuccess &&
-                   *blocks >= 1;
-        };
-        const bool req = s->nbuf_req >= 2 && s->nbuf_req <= kStMaxBuffers;
-        for (int G = std::min(v->max_threads / T, 15); G >= 1; --G) {
-            int blocks = 0;
-            int nb = req ? s->nbuf_req : 2;
-            if (!req && s->prec == PREC_F32 && fits(G, 3, &blocks)) nb = 3;
-            if (!fits(G, nb, &blocks)) continue;
+        if (stream_groups(s, v, &s->stream_G, &s->stream_nbuf, &s->stream_max_blocks)) {
             s->stream_v = v;
-            s->stream_G = G;
-            s->stream_nbuf = nb;
-            s->stream_max_blocks = blocks * s->num_sms;
             return true;
         }
     }
@@ -522,6 +559,7 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
             if (!choose_groups(v, (int)W, s->num_sms, G, maxb)) continue;
             s->variant = v;
             choose_stream(s, M, LIN, LOUT, SCALE);
+            choose_elem(s, M, LIN, LOUT, SCALE);
             s->R = R;
             s->W = (int)W;
             s->G = G;
@@ -721,10 +759,42 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
     const int64_t want = (rs.nsys + s->stream_G - 1) / s->stream_G;
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, s->stream_max_blocks));
     rs.nbuf = s->stream_nbuf;
-    v->launch(dim3((unsigned)grid), dim3(32 * v->W * s->stream_G), v->smem_bytes(s->stream_G, s->stream_nbuf), stream,
+    rs.groups = s->stream_G;
+    v->launch(dim3((unsigned)grid), dim3(v->threads(s->stream_G)), v->smem_bytes(s->stream_G, s->stream_nbuf), stream,
               &e->in, &e->out, op, rs);
     record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, s->stream_G, v->KL, v->KU, v->SV, v->LIN, v->LOUT, v->SCALE,
                   v->PREC, v->ALT, grid);
+    return true;
+}
+
+// Launch on the streaming kernel with element copies: no accumulation, full
+// output window, values aligned to their own size (packed complex ones to the
+// pair's).
+bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t stream)
+{
+    const StreamVariant* v = s->elem_v;
+    if (!v || io.accumulate || io.alt || io.oz0 > 0 || io.oz1 < io.M) return false;
+    // Few systems: the group kernel's short chunks give the lower latency as
+    // long as each of its resident groups solves at most two (N = 1 001 FP64:
+    // 592 systems 11.3 against 12.7 us, 1 184 systems 15.2 against 13.0;
+    // N = 501: 1 184 systems 10.9 against 11.7, 9 472 systems 37.4 against 25.3).
+    if (s->variant && io.nsys <= 2 * (int64_t)s->max_blocks * s->G) return false;
+    const int es = prec_f32_storage(v->PREC) ? 4 : 8;
+    const bool packed = v->LOUT == LAY_PACKED;
+    const uintptr_t in0 = reinterpret_cast<uintptr_t>(io.in) + (uintptr_t)io.in_off * es;
+    const uintptr_t out0 = reinterpret_cast<uintptr_t>(io.out) + (uintptr_t)io.out_off * es * (packed ? 2 : 1);
+    if (in0 % es || out0 % (packed ? 2 * es : es)) return false;
+    JwIO eio = io;
+    eio.nbuf = s->elem_nbuf;
+    eio.unit16 = in0 % 16 == 0 && (io.in_stride * es) % 16 == 0 &&
+                 (packed || (out0 % 16 == 0 && (io.out_stride * es) % 16 == 0));
+    const int64_t want = (io.nsys + s->elem_G - 1) / s->elem_G;
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, s->elem_max_blocks));
+    eio.groups = s->elem_G;
+    v->launch(dim3((unsigned)grid), dim3(v->threads(s->elem_G)), v->smem_bytes(s->elem_G, s->elem_nbuf), stream,
+              nullptr, nullptr, op, eio);
+    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, s->elem_G, v->KL, v->KU, v->SV, v->LIN, v->LOUT, v->SCALE,
+                  v->PREC, 0, grid);
     return true;
 }
 
@@ -736,6 +806,14 @@ PfSolveResult launch_jw_variant(AppState* s, const JwOperator& op, const JwIO& i
     if (launch_stream(s, op, io, stream)) {
         g_launches.fetch_add(1, std::memory_order_relaxed);
         g_stream_launches.fetch_add(1, std::memory_order_relaxed);
+        if (cudaPeekAtLastError() != cudaSuccess) {
+            cudaGetLastError();
+            return PFSOLVE_ERROR_FAILED_TO_LAUNCH_KERNEL;
+        }
+        return PFSOLVE_SUCCESS;
+    }
+    if (launch_elem(s, op, io, stream)) {
+        g_launches.fetch_add(1, std::memory_order_relaxed);
         if (cudaPeekAtLastError() != cudaSuccess) {
             cudaGetLastError();
             return PFSOLVE_ERROR_FAILED_TO_LAUNCH_KERNEL;
@@ -1542,6 +1620,10 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
         t.stream_G = cp.stream_G;
         t.stream_max_blocks = cp.stream_max_blocks;
         t.stream_nbuf = cp.stream_nbuf;
+        t.elem_v = cp.elem_v;
+        t.elem_G = cp.elem_G;
+        t.elem_max_blocks = cp.elem_max_blocks;
+        t.elem_nbuf = cp.elem_nbuf;
         return launch_jw_variant(&t, op, io, stream);
     }
     AppState t;
@@ -1561,7 +1643,8 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
     if (finish_variant(&t, M, LIN, LOUT, SCALE) != PFSOLVE_SUCCESS) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
     sj->chain_plans.push_back(AppState::ChainPlan{KL, KU, L.sv, LIN, LOUT, SCALE, t.variant, t.R, t.W, t.G,
                                                   t.max_blocks, t.stream_v, t.stream_G, t.stream_max_blocks,
-                                                  t.stream_nbuf});
+                                                  t.stream_nbuf, t.elem_v, t.elem_G, t.elem_max_blocks,
+                                                  t.elem_nbuf});
     return launch_jw_variant(&t, op, io, stream);
 }
 

@@ -145,6 +145,17 @@ struct StCfg {
     static_assert(CPLX ? (LOUT != LAY_REAL) : (LOUT == LAY_REAL), "layout pair");
 };
 
+// Threads of a CTA of G groups: at most kMaxThreads.  Where the table leaves
+// room for fewer than 256 threads' groups, further warps are launched that
+// only help to build it (a table of 4 096 tridiagonal rows took 128 threads
+// 40 us, 32 rows each) and exit before the first solve.  ALT builds two
+// tables in turn and keeps to its groups.
+template <class C>
+__host__ __device__ constexpr int st_threads(int G)
+{
+    return (C::T * G >= 256 || C::ALT) ? C::T * G : C::kMaxThreads;
+}
+
 // NB: staging buffers per group (2..kStMaxBuffers).
 template <class C>
 __host__ __device__ constexpr size_t st_fixed_bytes(int G, int NB)
@@ -381,7 +392,11 @@ __device__ void st_prologue(const JwOperator& op, typename C::CT* table, double*
     g.nthr = blockDim.x;
     g.bar_id = 1;
     g.seq = 0;
-    g.scratch = scratch_all;
+    // The scan over the CTA's warps exchanges through the table's own memory,
+    // which nothing writes before every warp has read the exchange: the
+    // scratch holds the groups' warps only.  (ALT's second scan comes after
+    // the first table is written.)
+    g.scratch = C::ALT ? scratch_all : reinterpret_cast<double*>(table);
     if constexpr (!C::ALT) {
         st_prologue_system<C>(op, 0, table, g);
         if constexpr (C::PRODS && (C::FWD || C::BWD)) {
@@ -432,13 +447,195 @@ __device__ void st_prologue(const JwOperator& op, typename C::CT* table, double*
     }
 }
 
-// ---- The kernel.
+// Shared-memory byte offset of swizzle row h of plane p of chunk c (of the
+// input and of the output layout) in the warp-major staging layout: the boxes
+// of warp c/32, then the next warp's; unit uu (< IB) of that row is at
+// + ((uu ^ swz(c)) << 4).
 template <class C>
-__global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_constant__ CUtensorMap tm_in,
-                                                                  const __grid_constant__ CUtensorMap tm_out,
-                                                                  const JwOperator op, const JwIO io)
+__device__ __forceinline__ size_t st_in_row(int p, int h, int c)
 {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
+    return ((size_t)(((c >> 5) * C::NPIN + p) * C::H + h) * 32 + (c & 31)) * C::ROWB;
+}
+template <class C>
+__device__ __forceinline__ size_t st_out_row(int p, int h, int c)
+{
+    return ((size_t)(((c >> 5) * C::NPOUT + p) * C::HO + h) * 32 + (c & 31)) * C::ROWBO;
+}
+
+// ---- How a group's systems reach its staging buffers and leave them.  NBUF
+// buffers per group, used in turn: system k of the group in buffer k mod NBUF,
+// its load issued NBUF - 1 systems ahead.  load(b, y) fills buffer b with
+// system y and completes one phase of its barrier; refill(b, y) does so once
+// the result that b held has left it; store(b, y) sends buffer b's result.
+//
+// TMA tensor copies: rows and strides of whole 16-byte units, R dividing M.
+// Lane 0 of each warp moves the warp's 32 chunks (x coordinates in storage
+// elements: 16 / ES per 16-byte unit).
+template <class C>
+struct StTma {
+    static constexpr int kArrivals = C::W;  // per barrier phase
+    const CUtensorMap *tm_in, *tm_out;
+    unsigned char* base;  // this group's buffers
+    uint64_t* bars;       // and their barriers
+    int wg, lane;
+    __device__ __forceinline__ unsigned char* buf(int b) const { return base + (size_t)b * C::BUF; }
+    __device__ __forceinline__ uint32_t bar(int b) const { return smem_u32(&bars[b]); }
+    __device__ __forceinline__ void load(int b, int64_t y) const
+    {
+        if (lane != 0) return;
+        mbar_arrive_expect_tx(bar(b), (uint32_t)(C::NPIN * C::H * 32 * C::ROWB));
+#pragma unroll
+        for (int p = 0; p < C::NPIN; ++p)
+#pragma unroll
+            for (int h = 0; h < C::H; ++h)
+                tma_load_3d(smem_u32(buf(b) + st_in_row<C>(p, h, 32 * wg)), tm_in, h * C::IB * (16 / C::ES), 32 * wg,
+                            (int)(C::CPLX ? 2 * y + p : y), bar(b));
+    }
+    __device__ __forceinline__ void refill(int b, int64_t y) const
+    {
+        if (lane == 0) {
+            bulk_wait_read_all();  // this warp's stores have been read out of shared memory
+            load(b, y);
+        }
+    }
+    __device__ __forceinline__ void store(int b, int64_t y) const
+    {
+        fence_proxy_async();
+        __syncwarp();
+        if (lane != 0) return;
+#pragma unroll
+        for (int p = 0; p < C::NPOUT; ++p)
+#pragma unroll
+            for (int h = 0; h < C::HO; ++h)
+                tma_store_3d(tm_out, h * C::IBO * (16 / C::ES), 32 * wg, (int)(C::NPOUT == 2 ? 2 * y + p : y),
+                             smem_u32(buf(b) + st_out_row<C>(p, h, 32 * wg)));
+        bulk_commit();
+    }
+    __device__ __forceinline__ void finish() const
+    {
+        if (lane == 0) bulk_wait_all();
+    }
+};
+
+// Element copies: any row count, stride and offset, into the same layout.
+// Consecutive lanes move consecutive 16-byte units (UNIT: rows, strides and
+// base all multiples of 16 bytes, only the row count is ragged) or single
+// values, by cp.async with zero-fill beyond the last row; the barrier counts
+// every lane's copies.  A copy instruction moves 512 (UNIT) or 32 ES bytes a
+// warp instead of a whole box: a few instructions a row, below what the solve
+// issues.  Measured, 268 MB of right-hand sides, against the group kernel that
+// took these launches before: FP64 N = 1 001 134 against 232 us, N = 201 127
+// against 259; mixed N = 1 001 264 against 540; FP32 N = 1 001 (134 MB) 102
+// against 194.  60 000 systems of 1 001 rows: 453 -> 242 us.
+template <class C>
+struct StElem {
+    static constexpr int kArrivals = C::T;
+    using Sto = typename C::Sto;
+    const JwIO* io;
+    unsigned char* base;
+    uint64_t* bars;
+    int wg, lane;
+    __device__ __forceinline__ unsigned char* buf(int b) const { return base + (size_t)b * C::BUF; }
+    __device__ __forceinline__ uint32_t bar(int b) const { return smem_u32(&bars[b]); }
+    // value q of this warp's 32 R (chunk q / R, row q % R of it)
+    __device__ __forceinline__ size_t in_at(int p, int q) const
+    {
+        const int c = q / C::R, j = q % C::R, u = j / C::EPU;
+        return st_in_row<C>(p, u / C::IB, 32 * wg + c) + (((u % C::IB) ^ swz_row<C::SWB>(c)) << 4) +
+               (j % C::EPU) * C::ES;
+    }
+    __device__ __forceinline__ size_t out_at(int p, int q) const
+    {
+        const int c = q / C::R, j = q % C::R, u = j / C::EPUO;
+        return st_out_row<C>(p, u / C::IBO, 32 * wg + c) + (((u % C::IBO) ^ swz_row<C::SWBO>(c)) << 4) +
+               (j % C::EPUO) * (16 / C::EPUO);
+    }
+    __device__ __forceinline__ void load(int b, int64_t y) const
+    {
+        constexpr int E = C::EPU;
+        const int M = (int)io->M, r0 = wg * 32 * C::R;
+        unsigned char* d = buf(b);
+#pragma unroll
+        for (int p = 0; p < C::NPIN; ++p) {
+            const Sto* src = reinterpret_cast<const Sto*>(io->in) + io->in_off +
+                             (C::CPLX ? 2 * y + p : y) * io->in_stride;
+            if (io->unit16) {
+#pragma unroll
+                for (int k = 0; k < C::R / E; ++k) {
+                    const int q = (32 * k + lane) * E, left = M - (r0 + q);
+                    cp_async16n(d + in_at(p, q), left > 0 ? src + r0 + q : src,
+                                left >= E ? 16 : (left > 0 ? left * C::ES : 0));
+                }
+            } else {
+#pragma unroll
+                for (int k = 0; k < C::R; ++k) {
+                    const int q = 32 * k + lane;
+                    const bool ok = r0 + q < M;
+                    cp_async_elem<Sto>(d + in_at(p, q), ok ? src + r0 + q : src, ok);
+                }
+            }
+        }
+        asm volatile("cp.async.mbarrier.arrive.noinc.shared::cta.b64 [%0];\n" ::"r"(bar(b)) : "memory");
+    }
+    __device__ __forceinline__ void refill(int b, int64_t y) const { load(b, y); }
+    __device__ __forceinline__ void store(int b, int64_t y) const
+    {
+        const int M = (int)io->M, r0 = wg * 32 * C::R;
+        const unsigned char* d = buf(b);
+        __syncwarp();
+        if constexpr (C::OPK) {  // packed complex values of 2 ES bytes
+            using S2 = typename Vec2Of<Sto>::type;
+            S2* dst = reinterpret_cast<S2*>(io->out) + io->out_off + y * io->out_stride;
+#pragma unroll
+            for (int k = 0; k < C::R; ++k) {
+                const int q = 32 * k + lane, row = r0 + q;
+                const S2 v = *reinterpret_cast<const S2*>(d + out_at(0, q));
+                if (row < M) dst[row] = v;
+            }
+        } else {
+            constexpr int E = C::EPU;
+#pragma unroll
+            for (int p = 0; p < C::NPOUT; ++p) {
+                Sto* dst = reinterpret_cast<Sto*>(io->out) + io->out_off +
+                           (C::NPOUT == 2 ? 2 * y + p : y) * io->out_stride;
+                if (io->unit16) {
+#pragma unroll
+                    for (int k = 0; k < C::R / E; ++k) {
+                        const int q = (32 * k + lane) * E, row = r0 + q;
+                        const float4 v = *reinterpret_cast<const float4*>(d + out_at(p, q));
+                        if (row + E <= M) {
+                            *reinterpret_cast<float4*>(dst + row) = v;
+                        } else {
+#pragma unroll
+                            for (int e = 0; e < E; ++e)
+                                if (row + e < M)
+                                    dst[row + e] = *reinterpret_cast<const Sto*>(d + out_at(p, q) + e * C::ES);
+                        }
+                    }
+                } else {
+#pragma unroll
+                    for (int k = 0; k < C::R; ++k) {
+                        const int q = 32 * k + lane, row = r0 + q;
+                        const Sto v = *reinterpret_cast<const Sto*>(d + out_at(p, q));
+                        if (row < M) dst[row] = v;
+                    }
+                }
+            }
+        }
+        __syncwarp();  // the buffer is the target of this warp's next load
+    }
+    __device__ __forceinline__ void finish() const { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+};
+
+// ---- A group's systems sys, sys + step, ... < nsys, solved with the CTA's
+// coefficient table.  The first NBUF - 1 of them are being loaded into the
+// buffers from bi on; bi and par (the phase parity of bi's barrier) are left
+// at the next system's.  Returns false when a completion wait ran out.
+template <class C, class LD>
+__device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, const typename C::CT* table, GroupCtx& g,
+                                       const LD& ld, const int NBUF, int64_t sys, const int64_t step,
+                                       const int64_t nsys, int& bi, uint32_t& par)
+{
     using V = typename C::V;
     using O = VOps<V>;
     using MS = typename C::MS;
@@ -447,76 +644,10 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_
     constexpr int R = C::R, W = C::W, T = C::T, U = C::U, NB = C::NB, S = C::S;
     constexpr int EPU = C::EPU, UD = C::UD, UO = C::UO, ES = C::ES;
     constexpr int KL = C::KLP, KU = C::KUP;  // staged halo rows (S times the band halo)
-    constexpr int IB = C::IB, H = C::H, IBO = C::IBO, HO = C::HO;
-    const int G = blockDim.x / T;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int grp = warp / W, wg = warp - grp * W;
-
-    CT* table = reinterpret_cast<CT*>(smem_raw);
-    double* scratch_all = reinterpret_cast<double*>(smem_raw + C::TBL);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::TBL + (size_t)G * W * kScratchPerWarp * sizeof(double));
-    // NBUF staging buffers per group, used in turn: system k of the group in
-    // buffer k mod NBUF, its load issued NBUF - 1 systems ahead.
-    const int NBUF = (io.nbuf >= 2 && io.nbuf <= kStMaxBuffers) ? io.nbuf : 2;
-    unsigned char* after = reinterpret_cast<unsigned char*>(bars + NBUF * G);
-    const uint32_t pad = (1024u - (smem_u32(after) & 1023u)) & 1023u;
-    unsigned char* buf_base = after + pad + (size_t)(NBUF * grp) * C::BUF;
-    auto buf_at = [&](int b) -> unsigned char* { return buf_base + (size_t)b * C::BUF; };
-    auto bar_at = [&](int b) -> uint32_t { return smem_u32(&bars[NBUF * grp + b]); };
-
-    // Shared-memory byte offset of swizzle row h of plane p of chunk c, in the
-    // warp-major staging layout (the boxes of warp c/32, then the next
-    // warp's); unit uu (< IB) of that row is at + ((uu ^ swz(c)) << 4).
-    constexpr int ROWB = C::ROWB, ROWBO = C::ROWBO;
-    auto in_row = [&](int p, int h, int c) -> size_t {
-        return ((size_t)(((c >> 5) * C::NPIN + p) * H + h) * 32 + (c & 31)) * ROWB;
-    };
-    auto out_row = [&](int p, int h, int c) -> size_t {
-        return ((size_t)(((c >> 5) * C::NPOUT + p) * HO + h) * 32 + (c & 31)) * ROWBO;
-    };
-    const int64_t nsys = io.nsys;
-    const int64_t step = (int64_t)gridDim.x * G;
-    int64_t sys = (int64_t)blockIdx.x * G + grp;
-
-    // lane 0 of each warp: load / store this warp's 32 chunks of one system
-    // (TMA x coordinates in storage elements: 16 / ES per 16-byte unit)
-    auto issue_load = [&](unsigned char* b, uint32_t bar, int64_t y) {
-        mbar_arrive_expect_tx(bar, (uint32_t)(C::NPIN * H * 32 * ROWB));
-#pragma unroll
-        for (int p = 0; p < C::NPIN; ++p)
-#pragma unroll
-            for (int h = 0; h < H; ++h)
-                tma_load_3d(smem_u32(b + in_row(p, h, 32 * wg)), &tm_in, h * IB * (16 / ES), 32 * wg,
-                            (int)(C::CPLX ? 2 * y + p : y), bar);
-    };
-    auto issue_store = [&](unsigned char* b, int64_t y) {
-#pragma unroll
-        for (int p = 0; p < C::NPOUT; ++p)
-#pragma unroll
-            for (int h = 0; h < HO; ++h)
-                tma_store_3d(&tm_out, h * IBO * (16 / ES), 32 * wg, (int)(C::NPOUT == 2 ? 2 * y + p : y),
-                             smem_u32(b + out_row(p, h, 32 * wg)));
-        bulk_commit();
-    };
-
-    if ((int)threadIdx.x < NBUF * G) mbar_init(smem_u32(&bars[threadIdx.x]), W);
-    mbar_init_fence();
-    __syncthreads();  // the barriers are initialised before any copy can complete on them
-    // The first system's copy does not depend on the coefficient table: it is
-    // in flight while the prologue reads the bands.
-    if (lane == 0)
-        for (int j = 0; j < NBUF - 1 && sys + j * step < nsys; ++j) issue_load(buf_at(j), bar_at(j), sys + j * step);
-    st_prologue<C>(op, table, scratch_all);
-    __syncthreads();
-
-    GroupCtx g;
-    g.lane = lane;
-    g.wg = wg;
-    g.W = W;
-    g.nthr = T;
-    g.bar_id = 1 + grp;
-    g.seq = 0;
-    g.scratch = scratch_all + (size_t)grp * W * kScratchPerWarp;
+    constexpr int IB = C::IB, IBO = C::IBO;
+    const int lane = g.lane, wg = g.wg;
+    auto in_row = [&](int p, int h, int c) -> size_t { return st_in_row<C>(p, h, c); };
+    auto out_row = [&](int p, int h, int c) -> size_t { return st_out_row<C>(p, h, c); };
 
     const int t = wg * 32 + lane;
     const int64_t s = (int64_t)t * R;
@@ -659,15 +790,13 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_
 
     const bool win_partial = io.iz0 > 0 || io.iz1 < io.M;
 
-    int bi = 0;        // buffer of this system
-    uint32_t par = 0;  // phase parity of its barrier
     for (; sys < nsys; sys += step) {
-        unsigned char* cur = buf_at(bi);
-        bool ok = mbar_wait_bounded(bar_at(bi), par);
+        unsigned char* cur = ld.buf(bi);
+        bool ok = mbar_wait_bounded(ld.bar(bi), par);
         ok = (W == 1) ? (__all_sync(FULL, ok) != 0) : group_and(g.bar_id, g.nthr, ok);
         if (!ok) {
-            if (threadIdx.x == 0) atomicOr(&g_stream_status, kStatusWaitTimeout);
-            break;
+            if (lane == 0) atomicOr(&g_stream_status, kStatusWaitTimeout);
+            return false;
         }
 
         // rows s-KL .. s+R+KU-1 of this system
@@ -758,13 +887,8 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_
         V (&x)[R + KL + KU] = be;
 
         // The load NBUF - 1 systems ahead goes into the buffer of the system
-        // before this one, once this warp's stores from it have been read out
-        // of shared memory.
-        if (sys + (NBUF - 1) * step < nsys && lane == 0) {
-            const int pb = (bi == 0) ? NBUF - 1 : bi - 1;
-            bulk_wait_read_all();
-            issue_load(buf_at(pb), bar_at(pb), sys + (NBUF - 1) * step);
-        }
+        // before this one.
+        if (sys + (NBUF - 1) * step < nsys) ld.refill((bi == 0) ? NBUF - 1 : bi - 1, sys + (NBUF - 1) * step);
 
         if constexpr (C::MIXED) {
             // x = M^{-1} g: FP32 solves of the residual, accumulated in FP64
@@ -1066,15 +1190,87 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_
                 }
             }
         }
-        fence_proxy_async();
-        __syncwarp();
-        if (lane == 0) issue_store(cur, sys);
+        ld.store(bi, sys);
         if (++bi == NBUF) {
             bi = 0;
             par ^= 1u;
         }
     }
-    if (lane == 0) bulk_wait_all();
+    return true;
+}
+
+// ---- The kernels: one CTA per SM, G groups, a table, every group its share of
+// the systems.
+template <class C, class LD>
+__device__ __forceinline__ void st_kernel(const JwOperator& op, const JwIO& io, LD ld)
+{
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using CT = typename C::CT;
+    constexpr int W = C::W, T = C::T;
+    const int G = io.groups;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int grp = warp / W, wg = warp - grp * W;
+    const bool solves = grp < G;  // else a helper warp (st_threads)
+    const int NBUF = (io.nbuf >= 2 && io.nbuf <= kStMaxBuffers) ? io.nbuf : 2;
+
+    CT* table = reinterpret_cast<CT*>(smem_raw);
+    double* scratch_all = reinterpret_cast<double*>(smem_raw + C::TBL);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(smem_raw + C::TBL + (size_t)G * W * kScratchPerWarp * sizeof(double));
+    unsigned char* after = reinterpret_cast<unsigned char*>(bars + NBUF * G);
+    const uint32_t pad = (1024u - (smem_u32(after) & 1023u)) & 1023u;
+    ld.base = after + pad + (size_t)(NBUF * grp) * C::BUF;
+    ld.bars = bars + NBUF * grp;
+    ld.wg = wg;
+    ld.lane = lane;
+    const int64_t nsys = io.nsys;
+    const int64_t step = (int64_t)gridDim.x * G;
+    const int64_t sys = (int64_t)blockIdx.x * G + grp;
+
+    if ((int)threadIdx.x < NBUF * G) mbar_init(smem_u32(&bars[threadIdx.x]), LD::kArrivals);
+    mbar_init_fence();
+    __syncthreads();  // the barriers are initialised before any copy can complete on them
+    // The first systems' copies do not depend on the coefficient table: they
+    // are in flight while the prologue reads the bands.
+    if (solves)
+        for (int j = 0; j < NBUF - 1 && sys + j * step < nsys; ++j) ld.load(j, sys + j * step);
+    st_prologue<C>(op, table, scratch_all);
+    __syncthreads();
+    if (!solves) return;
+
+    GroupCtx g;
+    g.lane = lane;
+    g.wg = wg;
+    g.W = W;
+    g.nthr = T;
+    g.bar_id = 1 + grp;
+    g.seq = 0;
+    g.scratch = scratch_all + (size_t)grp * W * kScratchPerWarp;
+    int bi = 0;
+    uint32_t par = 0;
+    st_run<C>(op, io, table, g, ld, NBUF, sys, step, nsys, bi, par);
+    ld.finish();
+}
+
+template <class C>
+__global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_constant__ CUtensorMap tm_in,
+                                                                  const __grid_constant__ CUtensorMap tm_out,
+                                                                  const JwOperator op, const JwIO io)
+{
+    StTma<C> ld;
+    ld.tm_in = &tm_in;
+    ld.tm_out = &tm_out;
+    st_kernel<C>(op, io, ld);
+}
+
+// Right-hand sides no tensor map describes: odd strides or offsets, row counts
+// that R does not divide.
+template <class C>
+__global__ void __launch_bounds__(C::kMaxThreads) jw_stream_elem_kernel(const JwOperator op,
+                                                                       const __grid_constant__ JwIO io)
+{
+    StElem<C> ld;
+    ld.io = &io;
+    st_kernel<C>(op, io, ld);
 }
 
 }  // namespace pfb

@@ -76,6 +76,8 @@ struct JwIO {
     int alt;                      // ALT mode: system 2y + h is the parity-h rows of row set y
     int plain;                    // long-system single pass: rows not 16-byte aligned, moved by plain loads/stores
     int nbuf;                     // streaming kernel: staging buffers per group (2..4; 0: 2)
+    int groups;                   // streaming kernel: groups per CTA
+    int unit16;                   // streaming kernel, element copies: rows, strides and bases in whole 16-byte units
 };
 
 // K consecutive steps in one kernel (numConsecutiveJWIterations = K).

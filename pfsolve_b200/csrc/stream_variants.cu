@@ -14,6 +14,14 @@ const StreamVariant* stream_variants_mixed(int* count);
 const StreamVariant* stream_variants_alt(int* count);
 const StreamVariant* stream_variants_f32(int* count);
 const StreamVariant* stream_variants_f32mem(int* count);
+const StreamVariant* stream_elem_f64(int* count);
+const StreamVariant* stream_elem_mixed(int* count);
+const StreamVariant* stream_elem_f32(int* count);
+const StreamVariant* stream_elem_f32mem(int* count);
+unsigned stream_elem_status_f64();
+unsigned stream_elem_status_mixed();
+unsigned stream_elem_status_f32();
+unsigned stream_elem_status_f32mem();
 unsigned stream_status_f64();
 unsigned stream_status_mixed();
 unsigned stream_status_alt();
@@ -21,16 +29,18 @@ unsigned stream_status_f32();
 unsigned stream_status_f32mem();
 
 const StreamVariant* find_stream_variant(int R, int W, int KL, int KU, int SV, int LIN, int LOUT, int SCALE, int PREC,
-                                         int ALT)
+                                         int ALT, int ELEM)
 {
     for (auto part : {stream_variants_f64, stream_variants_mixed, stream_variants_alt, stream_variants_f32,
-                      stream_variants_f32mem}) {
+                      stream_variants_f32mem, stream_elem_f64, stream_elem_mixed, stream_elem_f32,
+                      stream_elem_f32mem}) {
         int n = 0;
         const StreamVariant* vs = part(&n);
         for (int i = 0; i < n; ++i) {
             const StreamVariant& v = vs[i];
             if (v.R == R && v.W == W && v.KL == KL && v.KU == KU && v.SV == SV && v.LIN == LIN && v.LOUT == LOUT &&
-                v.SCALE == (SCALE ? 1 : 0) && v.PREC == PREC && v.ALT == (ALT ? 1 : 0))
+                v.SCALE == (SCALE ? 1 : 0) && v.PREC == PREC && v.ALT == (ALT ? 1 : 0) &&
+                v.ELEM == (ELEM ? 1 : 0))
                 return &v;
         }
     }
@@ -172,9 +182,14 @@ unsigned stream_status_fetch_clear()
     const unsigned a = stream_status_f64(), b = stream_status_mixed(), c = cluster_status_fetch_clear();
     const unsigned d = steps_status_fetch_clear(), e = batch_status_fetch_clear(), f = long_status_fetch_clear();
     const unsigned g = stream_status_alt(), h = stream_status_f32(), i = stream_status_f32mem();
-    if (a == ~0u || b == ~0u || c == ~0u || d == ~0u || e == ~0u || f == ~0u || g == ~0u || h == ~0u || i == ~0u)
-        return ~0u;
-    return a | b | c | d | e | f | g | h | i;
+    const unsigned ea = stream_elem_status_f64(), eb = stream_elem_status_mixed();
+    const unsigned ec = stream_elem_status_f32(), ed = stream_elem_status_f32mem();
+    unsigned all = 0;
+    for (unsigned v : {a, b, c, d, e, f, g, h, i, ea, eb, ec, ed}) {
+        if (v == ~0u) return ~0u;
+        all |= v;
+    }
+    return all;
 }
 
 }  // namespace pfb
