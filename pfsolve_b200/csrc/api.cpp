@@ -11,8 +11,10 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <functional>
 #include <map>
 #include <new>
+#include <queue>
 #include <tuple>
 #include <vector>
 
@@ -1695,6 +1697,8 @@ struct PfSolveBatch {
     int R = 8, W = 1, G = 1, spi = 64;
     int max_blocks = 0;
     const BatchVariant* variant = nullptr;
+    // real systems on the streaming solve; nullptr: the sweep or the group kernel
+    const BatchStreamVariant* bstream = nullptr;
     // sweep kernel (one system per lane) in use; nullptr: the group kernel
     const BatchSeqVariant* seq = nullptr;
     bool seq_ok = false;  // every entry allows the sweep kernel
@@ -1724,11 +1728,13 @@ void batch_drop_graph(PfSolveBatch* b)
     b->graph = nullptr;
 }
 
-PfSolveResult batch_build_items(PfSolveBatch* b, int spi)
+// spi systems per item, or per entry spi_of[e] systems of cost us_of[e] each.
+PfSolveResult batch_build_items(PfSolveBatch* b, int spi, const int* spi_of = nullptr, const double* us_of = nullptr)
 {
     b->items.clear();
     for (size_t e = 0; e < b->entries.size(); ++e) {
         const int64_t n = b->entries[e].io.nsys;
+        if (spi_of) spi = spi_of[e];  // per entry
         for (int64_t y0 = 0; y0 < n; y0 += spi) {
             WorkItem w;
             w.entry = (int)e;
@@ -1738,8 +1744,10 @@ PfSolveResult batch_build_items(PfSolveBatch* b, int spi)
             b->items.push_back(w);
         }
     }
-    // largest work first (bytes ~ rows x systems), ties by entry for locality
+    // largest work first (the given cost, else bytes ~ rows x systems), ties by
+    // entry for locality
     std::stable_sort(b->items.begin(), b->items.end(), [&](const WorkItem& x, const WorkItem& y) {
+        if (us_of) return us_of[x.entry] * (double)(x.y1 - x.y0) > us_of[y.entry] * (double)(y.y1 - y.y0);
         const int64_t cx = b->entries[x.entry].op.M * (x.y1 - x.y0);
         const int64_t cy = b->entries[y.entry].op.M * (y.y1 - y.y0);
         return cx > cy;
@@ -1814,6 +1822,7 @@ PfSolveResult batch_configure_seq(PfSolveBatch* b, int shape)
     b->seq = v;
     b->seq_shape = shape;
     b->variant = nullptr;
+    b->bstream = nullptr;
     b->R = 0;
     b->W = 0;
     b->G = v->NW;
@@ -1837,6 +1846,7 @@ PfSolveResult batch_configure(PfSolveBatch* b, int R)
         return PFSOLVE_ERROR_FAILED_TO_GET_ATTRIBUTE;
     b->variant = v;
     b->seq = nullptr;
+    b->bstream = nullptr;
     b->R = R;
     b->W = (int)W;
     b->G = G;
@@ -1844,10 +1854,101 @@ PfSolveResult batch_configure(PfSolveBatch* b, int R)
     return PFSOLVE_SUCCESS;
 }
 
+// Real systems of at most 2 048 rows on the streaming solve.  An item costs
+// one table build plus its systems, taken a round of a CTA's groups at a time;
+// the entries are cut into items of about equal cost: the cut whose greedy
+// schedule over the SMs (largest item first, as the device's queue hands them
+// out) ends earliest.
+PfSolveResult batch_configure_stream(PfSolveBatch* b)
+{
+    if (b->LIN != LAY_REAL || b->LOUT != LAY_REAL || b->SCALE || b->entries.empty() ||
+        b->Mmax > batch_stream_max_rows())
+        return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
+    const BatchStreamVariant* v = find_batch_stream_variant(b->KL, b->KU, b->SV, b->PREC);
+    if (!v || v->smem_bytes > 227 * 1024 || !allow_max_smem(v->func)) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
+    int blocks = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, v->func, 512, v->smem_bytes) != cudaSuccess ||
+        blocks < 1) {
+        cudaGetLastError();
+        return PFSOLVE_ERROR_FAILED_TO_GET_ATTRIBUTE;
+    }
+    for (const BatchEntryDev& e : b->entries)
+        if (e.io.accumulate) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
+    // Microseconds of an SM per system (batches that fill the chip; the mixed
+    // mode's, FP64 takes about 0.55 of them) and per table build, by the shape
+    // (padded rows 128, 256, 512, 1 024, 2 048) of an entry's groups.
+    static const double kSystemUs[5] = {0.13, 0.20, 0.40, 1.25, 2.40}, kBuildUs[5] = {7, 7, 8, 10, 13};
+    const double scale = b->PREC == PREC_MIXED ? 1.0 : 0.55;
+    auto system_us = [&](int64_t M) { return scale * kSystemUs[batch_stream_shape(M)]; };
+    double total = 0;
+    for (const BatchEntryDev& e : b->entries) total += (double)e.io.nsys * system_us(e.io.M);
+    std::vector<int> spi(b->entries.size()), best_spi;
+    std::vector<double> cost;
+    double best = 0;
+    for (double share = 0.5; share <= 8.0; share *= 1.0625) {
+        const double quantum = std::max(total / b->num_sms / share, 0.5);
+        cost.clear();
+        for (size_t e = 0; e < b->entries.size(); ++e) {
+            const JwIO& io = b->entries[e].io;
+            const int G = batch_stream_groups(io.M);
+            const double us = system_us(io.M), build = kBuildUs[batch_stream_shape(io.M)];
+            const int64_t rounds = (io.nsys + G - 1) / G;  // of the whole entry
+            const int64_t parts =
+                std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)std::ceil(io.nsys * us / quantum)));
+            const int64_t per = std::max<int64_t>(1, (rounds + parts - 1) / parts);
+            spi[e] = (int)std::min<int64_t>(per * G, INT32_MAX);
+            for (int64_t r = 0; r < rounds; r += per)
+                cost.push_back(build + (double)std::min(per, rounds - r) * G * us);
+        }
+        std::sort(cost.begin(), cost.end(), std::greater<double>());
+        std::priority_queue<double, std::vector<double>, std::greater<double>> busy;  // CTAs by when they are free
+        double end = 0;
+        for (double c : cost) {
+            double at = 0;
+            if ((int)busy.size() >= b->num_sms) {
+                at = busy.top();
+                busy.pop();
+            }
+            busy.push(at + c);
+            end = std::max(end, at + c);
+        }
+        if (best_spi.empty() || end < best) {
+            best = end;
+            best_spi = spi;
+        }
+    }
+    std::vector<double> us;
+    for (const BatchEntryDev& e : b->entries) us.push_back(system_us(e.io.M));
+    const PfSolveResult r = batch_build_items(b, 1, best_spi.data(), us.data());
+    if (r != PFSOLVE_SUCCESS) return r;
+    b->bstream = v;
+    b->seq = nullptr;
+    b->variant = nullptr;
+    b->R = 16;
+    b->W = (int)((b->Mmax + 511) / 512);
+    if (b->W == 3) b->W = 4;
+    b->G = 1;
+    b->max_blocks = b->num_sms;
+    b->spi = *std::max_element(best_spi.begin(), best_spi.end());
+    return PFSOLVE_SUCCESS;
+}
+
 PfSolveResult batch_launch(PfSolveBatch* b, cudaStream_t stream)
 {
     const int nitems = (int)b->items.size();
     if (nitems == 0) return PFSOLVE_SUCCESS;
+    if (b->bstream) {
+        const int grid = std::min(nitems, b->max_blocks);
+        if (nitems > grid && cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned int), stream) != cudaSuccess)
+            return PFSOLVE_ERROR_FAILED_TO_LAUNCH_KERNEL;
+        b->bstream->launch(dim3((unsigned)grid), stream, b->d_entries, b->d_items, nitems, b->d_counter);
+        g_launches.fetch_add(1, std::memory_order_relaxed);
+        if (cudaPeekAtLastError() != cudaSuccess) {
+            cudaGetLastError();
+            return PFSOLVE_ERROR_FAILED_TO_LAUNCH_KERNEL;
+        }
+        return PFSOLVE_SUCCESS;
+    }
     if (cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned int), stream) != cudaSuccess)
         return PFSOLVE_ERROR_FAILED_TO_LAUNCH_KERNEL;
     const int64_t want = (nitems + b->G - 1) / b->G;
@@ -1959,6 +2060,9 @@ PfSolveResult PfSolveBatchCreate(PfSolveBatch** out, CUdevice device, const PfSo
         d.io.nsys = en.nsys;
         d.io.M = en.M;
         d.io.accumulate = ((desc->block / 10) % 10) == 2;
+        // 16-byte units of a ragged row count (jw_batch_stream.cuh)
+        d.io.unit16 = reinterpret_cast<uintptr_t>(en.input) % 16 == 0 && en.inputStride % 2 == 0 &&
+                      reinterpret_cast<uintptr_t>(en.output) % 16 == 0 && en.outputStride % 2 == 0;
         b->entries.push_back(d);
         b->Mmax = std::max<int64_t>(b->Mmax, en.M);
     }
@@ -1989,6 +2093,11 @@ PfSolveResult PfSolveBatchCreate(PfSolveBatch** out, CUdevice device, const PfSo
         batch_configure_seq(b, 0) == PFSOLVE_SUCCESS) {
         PfSolveResult r = batch_build_items(b, 32);
         if (r != PFSOLVE_SUCCESS) return fail(r);
+        *out = b;
+        return PFSOLVE_SUCCESS;
+    }
+    // real systems of up to 2 048 rows: the streaming solve
+    if (!desc->rowsPerThread && desc->systemsPerItem <= 0 && batch_configure_stream(b) == PFSOLVE_SUCCESS) {
         *out = b;
         return PFSOLVE_SUCCESS;
     }
@@ -2057,6 +2166,7 @@ PfSolveResult PfSolveBatchAutotune(PfSolveBatch* b, cudaStream_t stream, int ite
     cudaEventCreate(&e1);
     double best = 1e300;
     int bestR = b->R, bestSpi = b->spi, bestShape = b->seq_shape;
+    bool bestStream = b->bstream != nullptr;  // the streaming solve, with its own item sizes
     auto time_shape = [&]() -> double {
         if (batch_launch(b, stream) != PFSOLVE_SUCCESS) return 1e300;  // warm-up
         cudaEventRecord(e0, stream);
@@ -2075,8 +2185,16 @@ PfSolveResult PfSolveBatchAutotune(PfSolveBatch* b, cudaStream_t stream, int ite
         if (per < best) {
             best = per;
             bestR = 0;
+            bestStream = false;
             bestSpi = 32;
             bestShape = shape;
+        }
+    }
+    if (batch_configure_stream(b) == PFSOLVE_SUCCESS) {
+        const double per = time_shape();
+        if (per < best) {
+            best = per;
+            bestStream = true;
         }
     }
     for (int R : {4, 8, 16, 2}) {
@@ -2088,13 +2206,15 @@ PfSolveResult PfSolveBatchAutotune(PfSolveBatch* b, cudaStream_t stream, int ite
                 best = per;
                 bestR = R;
                 bestSpi = spi;
+                bestStream = false;
             }
         }
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    PfSolveResult r = bestR ? batch_configure(b, bestR) : batch_configure_seq(b, bestShape);
-    if (r == PFSOLVE_SUCCESS) r = batch_build_items(b, bestSpi);
+    PfSolveResult r = bestStream ? batch_configure_stream(b)
+                                 : (bestR ? batch_configure(b, bestR) : batch_configure_seq(b, bestShape));
+    if (r == PFSOLVE_SUCCESS && !bestStream) r = batch_build_items(b, bestSpi);
     if (r == PFSOLVE_SUCCESS) b->tuned_ms = best;
     return r;
 }

@@ -33,6 +33,21 @@ struct BatchVariant {
 };
 const BatchVariant* find_batch_variant(int R, int KL, int KU, int SV, int LIN, int LOUT, int SCALE, int PREC);
 
+// Uneven batches of real systems on the streaming solve (jw_batch_stream.cuh):
+// one CTA an item, its groups shaped to the item's rows.
+struct BatchStreamVariant {
+    int KL, KU, SV, PREC;
+    const void* func;
+    size_t smem_bytes;
+    void (*launch)(dim3 grid, cudaStream_t st, const BatchEntryDev* entries, const WorkItem* items, int nitems,
+                   unsigned int* counter);
+};
+const BatchStreamVariant* find_batch_stream_variant(int KL, int KU, int SV, int PREC);
+int batch_stream_shape(int64_t M);            // 0 .. 4: padded rows 128, 256, 512, 1 024, 2 048
+int batch_stream_groups(int64_t M);           // systems a CTA solves at once
+int64_t batch_stream_max_rows();
+unsigned batch_stream_status_fetch_clear();
+
 // Uneven batches of bidiagonal steps (V*A within rows i-1..i+1, XXII in,
 // packed complex out, FP64): one complex system per lane, each system's rows
 // in one sweep, items of up to 32 systems per warp, NBUF chunks of 8 rows

@@ -185,7 +185,7 @@ unsigned stream_status_fetch_clear()
     const unsigned ea = stream_elem_status_f64(), eb = stream_elem_status_mixed();
     const unsigned ec = stream_elem_status_f32(), ed = stream_elem_status_f32mem();
     unsigned all = 0;
-    for (unsigned v : {a, b, c, d, e, f, g, h, i, ea, eb, ec, ed}) {
+    for (unsigned v : {a, b, c, d, e, f, g, h, i, ea, eb, ec, ed, batch_stream_status_fetch_clear()}) {
         if (v == ~0u) return ~0u;
         all |= v;
     }
