@@ -53,6 +53,11 @@ struct AppState {
     // tensor map describes
     const StreamVariant* elem_v = nullptr;
     int elem_G = 0, elem_max_blocks = 0, elem_nbuf = 2;
+    // both forms with real systems solved two at a time (nullptr: not compiled)
+    struct Pair {
+        const StreamVariant* v = nullptr;
+        int G = 0, max_blocks = 0, nbuf = 2;
+    } stream_pair, elem_pair;
     int stream_G = 0, stream_max_blocks = 0;
     int stream_nbuf = 2;  // staging buffers per group
     int nbuf_req = 0;     // caller's staging buffers per group (0: choose)
@@ -100,6 +105,7 @@ struct AppState {
         int stream_G, stream_max_blocks, stream_nbuf;
         const StreamVariant* elem_v;
         int elem_G, elem_max_blocks, elem_nbuf;
+        Pair stream_pair, elem_pair;
     };
     std::vector<ChainPlan> chain_plans;
     // streams
@@ -197,6 +203,16 @@ bool stream_groups(AppState* s, const StreamVariant* v, int* G_out, int* nbuf_ou
     return false;
 }
 
+// The form of a real streaming variant that solves systems two at a time.
+void choose_pair(AppState* s, const StreamVariant* v, AppState::Pair& out)
+{
+    out = AppState::Pair();
+    if (!v || v->LIN != LAY_REAL || v->ALT || v->SCALE) return;
+    const StreamVariant* p =
+        find_stream_variant(v->R, v->W, v->KL, v->KU, v->SV, LAY_XXII, LAY_XXII, 0, v->PREC, 0, v->ELEM);
+    if (p && stream_groups(s, p, &out.G, &out.nbuf, &out.max_blocks)) out.v = p;
+}
+
 // The streaming kernel with element copies for a plan that has a group-kernel
 // variant: launches whose rows no tensor map describes (odd strides or
 // offsets, row counts that the rows per thread do not divide) take it instead
@@ -205,14 +221,17 @@ bool stream_groups(AppState* s, const StreamVariant* v, int* G_out, int* nbuf_ou
 void choose_elem(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
 {
     s->elem_v = nullptr;
-    if ((s->prec != PREC_F64 && s->prec != PREC_MIXED && !prec_f32_storage(s->prec)) || s->no_stream || s->alt) return;
+    s->elem_pair = AppState::Pair();
+    if ((s->prec != PREC_F64 && s->prec != PREC_MIXED && !prec_f32_storage(s->prec)) || s->no_stream) return;
+    if (s->alt && s->prec != PREC_F64) return;
     static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 2}, {32, 4}};
     for (const auto& rw : shapes) {
         if (32 * (int64_t)rw[0] * rw[1] < M || (s->R_req && rw[0] != s->R_req)) continue;
         const StreamVariant* v =
-            find_stream_variant(rw[0], rw[1], s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, 0, 1);
+            find_stream_variant(rw[0], rw[1], s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, s->alt, 1);
         if (v && stream_groups(s, v, &s->elem_G, &s->elem_nbuf, &s->elem_max_blocks)) {
             s->elem_v = v;
+            choose_pair(s, v, s->elem_pair);
             break;
         }
     }
@@ -226,6 +245,7 @@ void choose_elem(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
 bool choose_stream(AppState* s, int64_t M, int LIN, int LOUT, int SCALE, bool alt = false)
 {
     s->stream_v = nullptr;
+    s->stream_pair = AppState::Pair();
     if ((s->prec != PREC_F64 && s->prec != PREC_MIXED && !prec_f32_storage(s->prec)) || s->no_stream) return false;
     int cand[3][2];
     int n = 0;
@@ -251,6 +271,7 @@ bool choose_stream(AppState* s, int64_t M, int LIN, int LOUT, int SCALE, bool al
         if (!v) continue;
         if (stream_groups(s, v, &s->stream_G, &s->stream_nbuf, &s->stream_max_blocks)) {
             s->stream_v = v;
+            choose_pair(s, v, s->stream_pair);
             return true;
         }
     }
@@ -514,6 +535,7 @@ PfSolveResult plan_alt(AppState* s, const PfSolveConfiguration& c, int base_prec
     // (partial output windows, unaligned rows) and kernelPath 1.
     s->no_stream = c.kernelPath == 1;
     if (s->prec == PREC_F64) choose_stream(s, M, LAY_REAL, LAY_REAL, 0, true);
+    choose_elem(s, M, LAY_REAL, LAY_REAL, 0);
     return PFSOLVE_SUCCESS;
 }
 
@@ -662,7 +684,7 @@ thread_local unsigned g_map_next = 0;
 bool same_io(const JwIO& a, const JwIO& b)
 {
     return a.in == b.in && a.out == b.out && a.in_off == b.in_off && a.in_stride == b.in_stride &&
-           a.out_off == b.out_off && a.out_stride == b.out_stride && a.nsys == b.nsys && a.M == b.M;
+           a.out_off == b.out_off && a.out_stride == b.out_stride && a.nsys == b.nsys && a.M == b.M && a.sets == b.sets;
 }
 
 const MapCacheEntry* row_maps(const void* key, int R, int LIN, int LOUT, int IB, int IBO, const JwIO& io, int es = 8)
@@ -747,6 +769,19 @@ PfSolveResult launch_long(AppState* s, const JwOperator& op, const JwIO& io, cud
     return PFSOLVE_SUCCESS;
 }
 
+// Real systems in pairs: one group solves systems 2y and 2y + 1 together, so
+// that every table value read from shared memory (the streaming kernel's bound
+// on real systems) serves two.  Worth it once every resident pair has two
+// rounds of work.
+bool take_pairs(const AppState::Pair& p, JwIO& io)
+{
+    if (!p.v || io.nsys < 4 * (int64_t)p.max_blocks * p.G) return false;
+    io.sets = io.nsys;
+    io.nsys = (io.nsys + 1) / 2;
+    io.nbuf = p.nbuf;
+    return true;
+}
+
 // Launch on the streaming variant when the plan has one and this launch's
 // buffers allow it (no accumulation, full output window, TMA-encodable rows).
 bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t stream)
@@ -756,16 +791,21 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
     // ALT: the launch counts systems (two per row set); the kernel, row sets
     JwIO rs = io;
     if (v->ALT) rs.nsys = io.nsys / 2;
+    int G = s->stream_G, max_blocks = s->stream_max_blocks;
+    rs.nbuf = s->stream_nbuf;
+    if (take_pairs(s->stream_pair, rs)) {
+        v = s->stream_pair.v;
+        G = s->stream_pair.G;
+        max_blocks = s->stream_pair.max_blocks;
+    }
     const MapCacheEntry* e = stream_maps(v, rs);
     if (!e) return false;
-    const int64_t want = (rs.nsys + s->stream_G - 1) / s->stream_G;
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, s->stream_max_blocks));
-    rs.nbuf = s->stream_nbuf;
-    rs.groups = s->stream_G;
-    v->launch(dim3((unsigned)grid), dim3(v->threads(s->stream_G)), v->smem_bytes(s->stream_G, s->stream_nbuf), stream,
-              &e->in, &e->out, op, rs);
-    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, s->stream_G, v->KL, v->KU, v->SV, v->LIN, v->LOUT, v->SCALE,
-                  v->PREC, v->ALT, grid);
+    const int64_t want = (rs.nsys + G - 1) / G;
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, max_blocks));
+    rs.groups = G;
+    v->launch(dim3((unsigned)grid), dim3(v->threads(G)), v->smem_bytes(G, rs.nbuf), stream, &e->in, &e->out, op, rs);
+    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, G, v->KL, v->KU, v->SV, s->stream_v->LIN, s->stream_v->LOUT,
+                  v->SCALE, v->PREC, v->ALT, grid);
     return true;
 }
 
@@ -775,7 +815,7 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
 bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t stream)
 {
     const StreamVariant* v = s->elem_v;
-    if (!v || io.accumulate || io.alt || io.oz0 > 0 || io.oz1 < io.M) return false;
+    if (!v || io.accumulate || io.oz0 > 0 || io.oz1 < io.M) return false;
     // Few systems: the group kernel's short chunks give the lower latency as
     // long as each of its resident groups solves at most two (N = 1 001 FP64:
     // 592 systems 11.3 against 12.7 us, 1 184 systems 15.2 against 13.0;
@@ -787,16 +827,23 @@ bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t
     const uintptr_t out0 = reinterpret_cast<uintptr_t>(io.out) + (uintptr_t)io.out_off * es * (packed ? 2 : 1);
     if (in0 % es || out0 % (packed ? 2 * es : es)) return false;
     JwIO eio = io;
+    if (v->ALT) eio.nsys = io.nsys / 2;  // row sets, two systems each
     eio.nbuf = s->elem_nbuf;
     eio.unit16 = in0 % 16 == 0 && (io.in_stride * es) % 16 == 0 &&
                  (packed || (out0 % 16 == 0 && (io.out_stride * es) % 16 == 0));
-    const int64_t want = (io.nsys + s->elem_G - 1) / s->elem_G;
-    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, s->elem_max_blocks));
-    eio.groups = s->elem_G;
-    v->launch(dim3((unsigned)grid), dim3(v->threads(s->elem_G)), v->smem_bytes(s->elem_G, s->elem_nbuf), stream,
-              nullptr, nullptr, op, eio);
-    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, s->elem_G, v->KL, v->KU, v->SV, v->LIN, v->LOUT, v->SCALE,
-                  v->PREC, 0, grid);
+    int G = s->elem_G, max_blocks = s->elem_max_blocks;
+    if (take_pairs(s->elem_pair, eio)) {
+        v = s->elem_pair.v;
+        G = s->elem_pair.G;
+        max_blocks = s->elem_pair.max_blocks;
+    }
+    const int64_t want = (eio.nsys + G - 1) / G;
+    const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, max_blocks));
+    eio.groups = G;
+    v->launch(dim3((unsigned)grid), dim3(v->threads(G)), v->smem_bytes(G, eio.nbuf), stream, nullptr, nullptr, op,
+              eio);
+    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, G, v->KL, v->KU, v->SV, s->elem_v->LIN, s->elem_v->LOUT,
+                  v->SCALE, v->PREC, v->ALT, grid);
     return true;
 }
 
@@ -1626,6 +1673,8 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
         t.elem_G = cp.elem_G;
         t.elem_max_blocks = cp.elem_max_blocks;
         t.elem_nbuf = cp.elem_nbuf;
+        t.stream_pair = cp.stream_pair;
+        t.elem_pair = cp.elem_pair;
         return launch_jw_variant(&t, op, io, stream);
     }
     AppState t;
@@ -1646,7 +1695,7 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
     sj->chain_plans.push_back(AppState::ChainPlan{KL, KU, L.sv, LIN, LOUT, SCALE, t.variant, t.R, t.W, t.G,
                                                   t.max_blocks, t.stream_v, t.stream_G, t.stream_max_blocks,
                                                   t.stream_nbuf, t.elem_v, t.elem_G, t.elem_max_blocks,
-                                                  t.elem_nbuf});
+                                                  t.elem_nbuf, t.stream_pair, t.elem_pair});
     return launch_jw_variant(&t, op, io, stream);
 }
 

@@ -77,7 +77,8 @@ struct StCfg {
     // Coefficient table planes, each one CT2 per (row pair, thread).
     // FP64 / FP32: NB weights (scaled by the LU pivots), -l, -h, Scale factor.
     // Mixed: NB weights (unscaled), the solve's sub- and super-diagonal in FP64
-    // (residual), FP32 packs {m, m', -l, -l'} and {-h, -h', 0, 0}, Scale factor.
+    // (residual), FP32 packs {m, m', -l, -l'} and {-h, -h'} (8-byte entries, the
+    // first half of their plane), Scale factor.
     // FP32 arithmetic, 16 or 32 rows per thread (QUAD): one float4 per (row
     // quad, thread), and two more planes, the products of -l over the chunk's
     // rows up to each row and of -h from each row on, so that a system's
@@ -366,10 +367,9 @@ __device__ void st_prologue_system(const JwOperator& op, int h, typename C::CT* 
                 if constexpr (C::BWD) put(C::P_CU, cu);
                 put32(C::P_F1, 0, m);
                 put32(C::P_F1, 2, nl);
-                if constexpr (C::BWD) {
-                    put32(C::P_F2, 0, nh);
-                    put32(C::P_F2, 2, 0.0);
-                }
+                if constexpr (C::BWD)
+                    reinterpret_cast<float*>(table + (size_t)C::P_F2 * U * C::TP * 2)[((jj >> 1) * C::TP + tt) * 2 +
+                                                                                     (jj & 1)] = (float)nh;
             } else {
                 if constexpr (C::FWD) put(C::P_NL, nl);
                 if constexpr (C::BWD) put(C::P_NH, nh);
@@ -553,12 +553,14 @@ struct StElem {
     __device__ __forceinline__ void load(int b, int64_t y) const
     {
         constexpr int E = C::EPU;
-        const int M = (int)io->M, r0 = wg * 32 * C::R;
+        const int r0 = wg * 32 * C::R;
         unsigned char* d = buf(b);
 #pragma unroll
         for (int p = 0; p < C::NPIN; ++p) {
-            const Sto* src = reinterpret_cast<const Sto*>(io->in) + io->in_off +
-                             (C::CPLX ? 2 * y + p : y) * io->in_stride;
+            const int64_t set = C::CPLX ? 2 * y + p : y;
+            // (real systems in pairs: an odd last one has no partner)
+            const int M = (C::CPLX && io->sets && set >= io->sets) ? 0 : (int)io->M;
+            const Sto* src = reinterpret_cast<const Sto*>(io->in) + io->in_off + (M ? set : 0) * io->in_stride;
             if (io->unit16) {
 #pragma unroll
                 for (int k = 0; k < C::R / E; ++k) {
@@ -596,6 +598,7 @@ struct StElem {
             constexpr int E = C::EPU;
 #pragma unroll
             for (int p = 0; p < C::NPOUT; ++p) {
+                if (C::NPOUT == 2 && io->sets && 2 * y + p >= io->sets) break;
                 Sto* dst = reinterpret_cast<Sto*>(io->out) + io->out_off +
                            (C::NPOUT == 2 ? 2 * y + p : y) * io->out_stride;
                 if (io->unit16) {
@@ -655,24 +658,22 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
     auto coef = [&](int p, int u) -> CT2 { return tb[(p * U + u) * C::TP]; };
 
     auto coef4 = [&](int p, int u) -> float4 { return reinterpret_cast<const float4*>(tb)[(p * U + u) * C::TP]; };
-    // Mixed precision, real systems of up to 16 rows per thread: the FP32 solve
-    // factors {m, -l} stay in registers for the whole kernel (every refinement
-    // sweep reuses them); {-h} too for up to 8 rows per thread (at 16, the
-    // 128-register bound of a 512-thread CTA leaves no room for them).
-    constexpr bool kHoist = C::MIXED && !C::CPLX && U <= 8;
-    constexpr bool kHoist2 = kHoist && U <= 4;
+    // Mixed precision, up to 16 rows per thread: the FP32 solve factors {m, -l}
+    // stay in registers for the whole kernel (every refinement sweep reuses
+    // them); {-h} too for up to 8 rows per thread
+    // (at 16, the 128-register bound of a 512-thread CTA leaves no room for
+    // them); under a 256-thread bound both, up to 16 rows per thread.
+    constexpr bool kWide = C::kMaxThreads <= 256;
+    constexpr bool kHoist = C::MIXED && U <= 8 && (!C::CPLX || kWide);
+    constexpr bool kHoist2 = kHoist && (U <= 4 || kWide);
+    const float2* f2p = reinterpret_cast<const float2*>(table + (size_t)C::P_F2 * U * C::TP * 2) + t;
     float4 hf1[kHoist ? U : 1];
     float2 hf2[kHoist2 ? U : 1];
     if constexpr (kHoist) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             hf1[u] = coef4(C::P_F1, u);
-            if constexpr (kHoist2 && C::BWD) {
-                const float4 f = coef4(C::P_F2, u);
-                hf2[u] = make_float2(f.x, f.y);
-            } else if constexpr (kHoist2) {
-                hf2[u] = make_float2(0.0f, 0.0f);
-            }
+            if constexpr (kHoist2) hf2[u] = C::BWD ? f2p[u * C::TP] : make_float2(0.0f, 0.0f);
         }
     }
     auto F1 = [&](int u) -> float4 {
@@ -680,12 +681,8 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
         else return coef4(C::P_F1, u);
     };
     auto F2 = [&](int u) -> float2 {
-        if constexpr (kHoist2) {
-            return hf2[u];
-        } else {
-            const float4 f = coef4(C::P_F2, u);
-            return make_float2(f.x, f.y);
-        }
+        if constexpr (kHoist2) return hf2[u];
+        else return f2p[u * C::TP];
     };
 
     // Scan multipliers: products of -l and -h over this thread's chunk (in the
@@ -743,7 +740,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
     if constexpr (C::BWD && C::MIXED) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const float4 c = coef4(C::P_F2, u);
+            const float2 c = F2(u);
             Ab32 = c.x * Ab32;
             Ab32 = c.y * Ab32;
         }
@@ -966,9 +963,12 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
                     }
                 }
                 if constexpr (C::BWD) {
+                    float2 fb[U];  // read once a sweep
+#pragma unroll
+                    for (int u = 0; u < U; ++u) fb[u] = F2(u);
 #pragma unroll
                     for (int u = U - 1; u >= 0; --u) {
-                        const float2 f = F2(u);
+                        const float2 f = fb[u];
                         if (u < U - 1) d[2 * u + 1] = OF::fma(f.y, d[2 * u + 2], d[2 * u + 1]);
                         d[2 * u] = OF::fma(f.x, d[2 * u + 1], d[2 * u]);
                     }
@@ -978,7 +978,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
                     float p = 1.0f;
 #pragma unroll
                     for (int u = U - 1; u >= 0; --u) {
-                        const float2 f = F2(u);
+                        const float2 f = fb[u];
                         p = f.y * p;
                         d[2 * u + 1] = OF::fma(p, q, d[2 * u + 1]);
                         p = f.x * p;

@@ -77,6 +77,7 @@ struct JwIO {
     int plain;                    // long-system single pass: rows not 16-byte aligned, moved by plain loads/stores
     int nbuf;                     // streaming kernel: staging buffers per group (2..4; 0: 2)
     int groups;                   // streaming kernel: groups per CTA
+    int64_t sets;                 // real systems solved in pairs as XXII ones: their number (0: 2 nsys row sets)
     int unit16;                   // streaming kernel, element copies: rows, strides and bases in whole 16-byte units
 };
 

@@ -70,6 +70,17 @@ inline void st_elem_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t s
                   StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>::IBO,                         \
                   &st_launch_fn<StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>>, 1,               \
                   &st_threads_fn<StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>>}
+// ALT by element copies: row sets of M <= 256, 512, 1024, 2048 and 4096 rows
+#define PFB_SVAE(R, W, KL, KU, SV)                                                                             \
+    StreamVariant{R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64,                                      \
+                  StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>::kMaxThreads,                \
+                  (const void*)&jw_stream_elem_kernel<StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>>, \
+                  &st_smem_fn<StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>>, 0, 0,           \
+                  &st_elem_launch_fn<StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>>, 1,      \
+                  &st_threads_fn<StCfg<R, W, KL, KU, SV, LAY_REAL, LAY_REAL, false, PREC_F64, 1>>, 1}
+#define PFB_SALTE(KL, KU, SV)                                                                                 \
+    PFB_SVAE(8, 1, KL, KU, SV), PFB_SVAE(16, 1, KL, KU, SV), PFB_SVAE(16, 2, KL, KU, SV), PFB_SVAE(16, 4, KL, KU, SV), \
+        PFB_SVAE(32, 4, KL, KU, SV)
 // 8, 16 and 32 rows per thread, 1, 2 and 4 warps per row set (M <= 4096)
 #define PFB_SALT(KL, KU, SV)                                                                                  \
     PFB_SVA(8, 1, KL, KU, SV), PFB_SVA(8, 2, KL, KU, SV), PFB_SVA(8, 4, KL, KU, SV), PFB_SVA(16, 1, KL, KU, SV), \
@@ -89,7 +100,10 @@ inline void st_elem_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t s
     PFB_SVP(16, 1, KL, KU, SV, LAY_XXII, LAY_PACKED, SC, P), PFB_SVP(16, 2, KL, KU, SV, LAY_XXII, LAY_PACKED, SC, P), \
         PFB_SVP(32, 1, KL, KU, SV, LAY_XXII, LAY_PACKED, SC, P), PFB_SVP(32, 2, KL, KU, SV, LAY_XXII, LAY_PACKED, SC, P)
 #define PFB_SCPLX(KL, KU, SV, SC) PFB_SCPLXP(KL, KU, SV, SC, PREC_F64)
-
+// real systems two at a time, as XXII complex ones (a pair shares every table
+// read): by tensor copies and by element copies
+#define PFB_SPAIR(R, W, KL, KU, SV, P)                                                                          \
+    PFB_SVP(R, W, KL, KU, SV, LAY_XXII, LAY_XXII, false, P), PFB_SVE(R, W, KL, KU, SV, LAY_XXII, LAY_XXII, false, P)
 
 // Status word of this translation unit's kernels: read and clear.
 #define PFB_STREAM_STATUS_ACCESSOR(name)                                          \

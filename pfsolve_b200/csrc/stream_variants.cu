@@ -15,13 +15,21 @@ const StreamVariant* stream_variants_alt(int* count);
 const StreamVariant* stream_variants_f32(int* count);
 const StreamVariant* stream_variants_f32mem(int* count);
 const StreamVariant* stream_elem_f64(int* count);
+const StreamVariant* stream_pair_f64(int* count);
 const StreamVariant* stream_elem_mixed(int* count);
+const StreamVariant* stream_pair_mixed(int* count);
 const StreamVariant* stream_elem_f32(int* count);
+const StreamVariant* stream_pair_f32(int* count);
 const StreamVariant* stream_elem_f32mem(int* count);
+const StreamVariant* stream_pair_f32mem(int* count);
 unsigned stream_elem_status_f64();
+unsigned stream_pair_status_f64();
 unsigned stream_elem_status_mixed();
+unsigned stream_pair_status_mixed();
 unsigned stream_elem_status_f32();
+unsigned stream_pair_status_f32();
 unsigned stream_elem_status_f32mem();
+unsigned stream_pair_status_f32mem();
 unsigned stream_status_f64();
 unsigned stream_status_mixed();
 unsigned stream_status_alt();
@@ -33,7 +41,7 @@ const StreamVariant* find_stream_variant(int R, int W, int KL, int KU, int SV, i
 {
     for (auto part : {stream_variants_f64, stream_variants_mixed, stream_variants_alt, stream_variants_f32,
                       stream_variants_f32mem, stream_elem_f64, stream_elem_mixed, stream_elem_f32,
-                      stream_elem_f32mem}) {
+                      stream_elem_f32mem, stream_pair_f64, stream_pair_mixed, stream_pair_f32, stream_pair_f32mem}) {
         int n = 0;
         const StreamVariant* vs = part(&n);
         for (int i = 0; i < n; ++i) {
@@ -107,13 +115,13 @@ bool encode_row_maps(int R_, int LIN, int LOUT, int IB, int IBO, const JwIO& io,
     if (M % R != 0 || io.nsys < 1) return false;
     const int64_t chunks = M / R;
     const bool cplx = LIN != LAY_REAL;
-    const int64_t sets = cplx ? 2 * io.nsys : io.nsys;
+    const int64_t sets = cplx ? (io.sets ? io.sets : 2 * io.nsys) : io.nsys;
     const char* in0 = reinterpret_cast<const char*>(io.in) + io.in_off * es;
     char* out0 = reinterpret_cast<char*>(io.out);
     if (!encode_rows(in, in0, R, chunks, sets, io.in_stride * es, IB, es)) return false;
     if (LOUT == LAY_PACKED)  // complex elements of 2 es bytes: 2 R storage elements per chunk
         return encode_rows(out, out0 + io.out_off * 2 * es, 2 * R, chunks, io.nsys, io.out_stride * 2 * es, IBO, es);
-    const int64_t osets = (LOUT == LAY_XXII) ? 2 * io.nsys : io.nsys;
+    const int64_t osets = (LOUT == LAY_XXII) ? sets : io.nsys;
     return encode_rows(out, out0 + io.out_off * es, R, chunks, osets, io.out_stride * es, IBO, es);
 }
 
@@ -185,7 +193,8 @@ unsigned stream_status_fetch_clear()
     const unsigned ea = stream_elem_status_f64(), eb = stream_elem_status_mixed();
     const unsigned ec = stream_elem_status_f32(), ed = stream_elem_status_f32mem();
     unsigned all = 0;
-    for (unsigned v : {a, b, c, d, e, f, g, h, i, ea, eb, ec, ed, batch_stream_status_fetch_clear()}) {
+    for (unsigned v : {a, b, c, d, e, f, g, h, i, ea, eb, ec, ed, batch_stream_status_fetch_clear(), stream_pair_status_f64(),
+                       stream_pair_status_mixed(), stream_pair_status_f32(), stream_pair_status_f32mem()}) {
         if (v == ~0u) return ~0u;
         all |= v;
     }

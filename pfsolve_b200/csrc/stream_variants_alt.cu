@@ -13,6 +13,14 @@ static const StreamVariant kPart[] = {
     PFB_SALT(1, 0, SV_UPPER),
     PFB_SALT(1, 0, SV_NONE),
     PFB_SALT(0, 0, SV_UPPER),
+    // by element copies
+    PFB_SALTE(0, 0, SV_TRI),
+    PFB_SALTE(0, 1, SV_LOWER),
+    PFB_SALTE(0, 1, SV_NONE),
+    PFB_SALTE(0, 0, SV_LOWER),
+    PFB_SALTE(1, 0, SV_UPPER),
+    PFB_SALTE(1, 0, SV_NONE),
+    PFB_SALTE(0, 0, SV_UPPER),
 };
 
 const StreamVariant* stream_variants_alt(int* count)

@@ -100,3 +100,28 @@ def test_complex_chain_odd_rows(M, block, lshift):
     got = out[:2 * M * Y].reshape(Y, 2 * M)
     assert (np.linalg.norm(got - ref, axis=1) / np.linalg.norm(ref, axis=1)).max() <= TOL["f64"]
     assert (out[2 * M * Y:] == 0).all()
+
+
+@pytest.mark.parametrize("M", [100, 255, 500, 999, 1001, 2047, 4095])
+def test_alt_odd_row_sets(M):
+    """ALT mode by element copies: row counts the streaming kernel's chunks do
+    not divide, odd strides."""
+    import torch
+
+    from pfsolve_b200.api import App, last_launch
+    B = 9001 if M < 512 else 2401
+    for ub, jwt in [(2, 113), (1, 110), (0, 113), (0, 111)]:
+        rng = np.random.default_rng(M + ub + jwt)
+        bands = WL.alt_bands(rng, M, ub)
+        case = O.Case(M=M, batch=B, upperBanded=ub, jw_type=jwt, bitmask=capi.RUNTIME_SCALEC, run_scaleC=0.5)
+        rhs = rng.uniform(-1, 1, case.rhs_len())
+        tb, to = torch.from_numpy(bands).cuda(), torch.from_numpy(rhs.copy()).cuda()
+        app = App(buffer=tb, outputBuffer=to, **J.case_fields(case))
+        app.append(**J.launch_fields(case))
+        torch.cuda.synchronize()
+        info = last_launch()
+        assert (info["kernel"], info["alt"]) == (capi.PFSOLVE_KERNEL_STREAMING, 1)
+        x = to.cpu().numpy()
+        app.close()
+        ref = O.jw_step_alt(case, bands, rhs, nthreads=16)
+        assert np.abs(x - ref).max() <= 1e-13 * np.abs(ref).max(), (ub, jwt)
