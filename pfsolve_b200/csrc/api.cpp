@@ -944,6 +944,7 @@ PfSolveResult append_steps(PfSolveApplication* app, const PfSolveLaunchParams* l
         d.bands = static_cast<const double*>(b);
         step_layout(c, k, s->K, d);
         d.perm_r = s->steps_r;
+        d.perm_mul = fast_div_mul(s->steps_r);
         d.perm_m = d.M % d.perm_r;
         d.perm_ceil = (d.M + d.perm_r - 1) / d.perm_r;
         d.perm_floor = d.M / d.perm_r;
@@ -970,7 +971,9 @@ PfSolveResult append_steps(PfSolveApplication* app, const PfSolveLaunchParams* l
         const int nw = (int)std::max<int64_t>(1, (nblk + (int64_t)s->num_sms * rounds - 1) / ((int64_t)s->num_sms * rounds));
         const int64_t grid = std::min<int64_t>(s->num_sms, (nblk + nw - 1) / nw);
         const int64_t Mtab = c.upperBanded ? S.M_in : S.M_out;
-        s->seq_v->launch(dim3((unsigned)grid), dim3(32 * nw), seq_steps_smem_bytes(S.K, Mtab, nw, s->seq_v->CH), stream,
+        // few sweeping warps: more that only help to build the step tables
+        io.groups = nw;
+        s->seq_v->launch(dim3((unsigned)grid), dim3(32 * std::max(nw, 12)), seq_steps_smem_bytes(S.K, Mtab, nw, s->seq_v->CH), stream,
                          &tin, &tout,
                          S, io);
         g_launches.fetch_add(1, std::memory_order_relaxed);

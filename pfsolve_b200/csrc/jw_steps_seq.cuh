@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
     constexpr int CS = CH == 16 ? 4 : 3;        // chunk of a sweep position: >> CS
     constexpr int ROWB = CH * 8;                // bytes of a system's row in a box
     constexpr int KMAX = K;
-    const int NW = blockDim.x >> 5;
+    const int NW = io.groups;  // sweeping warps; any others only help with the table
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int M0 = (int)S.M_in, Mout = (int)S.M_out;
     const int Mtab = UB ? M0 : Mout;  // rows of the widest step
@@ -95,17 +95,28 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + seq_table_bytes(K, Mtab) + (size_t)NW * kSeqBufs * kSeqBufBytes) +
                      warp * kSeqBufs;
 
-    // ---- coefficient table (rows at or beyond a step's M_s are never read)
+    // ---- coefficient table (rows at or beyond a step's M_s are never read).
+    // Four entries' loads in flight a thread, positions by reciprocal, and at
+    // least 12 warps at work: 2 048 systems of 512 rows (one sweeping warp an
+    // SM) took 66 us at K = 4 and 115 at K = 8 with the sweeping warps alone,
+    // and take 41.5 and 66.
     // the step that applies the matvec diagonal (JwStepDesc.diag)
     constexpr int dstep = MV ? (UB ? 0 : K - 1) : -1;
+#pragma unroll 4
     for (int e = threadIdx.x; e < K * Mtab; e += blockDim.x) {
-        const int s = e / Mtab, i = e - s * Mtab;
+        int s = 0, i = e;  // step and row
+#pragma unroll
+        for (int q = 1; q < K; ++q)
+            if (e >= q * Mtab) {
+                s = q;
+                i = e - q * Mtab;
+            }
         const JwStepDesc& d = S.st[s];
         double o = 0.0, q = 0.0, dv = 1.0;
         if (i < d.M) {
             int pos = i;
             if (S.perm) {
-                const int r = (int)d.perm_r, t = i / r, j = i - t * r, m = (int)d.perm_m;
+                const int r = (int)d.perm_r, t = (int)fast_div((unsigned)i, d.perm_mul), j = i - t * r, m = (int)d.perm_m;
                 pos = t + ((j < m) ? j * (int)d.perm_ceil : m * (int)d.perm_ceil + (j - m) * (int)d.perm_floor);
             }
             if (MV) {
@@ -120,9 +131,10 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
         tabA[e] = make_double2(o, q);
         if (s == dstep) tabD[i] = dv;
     }
-    if (lane < kSeqBufs) mbar_init(smem_u32(&bars[lane]), 1);
+    if (warp < NW && lane < kSeqBufs) mbar_init(smem_u32(&bars[lane]), 1);
     mbar_init_fence();
     __syncthreads();
+    if (warp >= NW) return;
 
     // ---- sweep geometry (sweep position p <-> row): ascending p = row;
     // descending p = R0 - row with R0 the top row of the top chunk.  At sweep
@@ -154,7 +166,11 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
         asm volatile("ld.shared.v2.f64 {%0, %1}, [%2];\n" : "=d"(v.x), "=d"(v.y) : "r"(a));
         return v;
     };
-    auto sts = [](uint32_t a, double v) { asm volatile("st.shared.f64 [%0], %1;\n" ::"r"(a), "d"(v) : "memory"); };
+    // Results go to staged rows that only this lane's ordered (volatile)
+    // accesses touch before the chunk's store, so the store claims no other
+    // memory: the coefficient reads below it, plain loads of a table that never
+    // changes, may move above it.
+    auto sts = [](uint32_t a, double v) { asm volatile("st.shared.f64 [%0], %1;\n" ::"r"(a), "d"(v)); };
     // byte offset of box row rb (0 .. CH-1) of this lane's system in a buffer
     auto lane_off = [&](int rb) -> uint32_t {
         return (uint32_t)(lane * ROWB + ((((rb >> 1) ^ sw)) << 4) + ((rb & 1) << 3));
@@ -186,8 +202,6 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
             bulk_commit();
         }
     };
-    const uint32_t tabA_u = smem_u32(tabA), tabD_u = smem_u32(tabD);
-
     for (int64_t blk = (int64_t)blockIdx.x * NW + warp; blk < nblk && ok; blk += (int64_t)gridDim.x * NW) {
         const int sys0 = (int)(blk * 32);
         if (lane == 0) {
@@ -240,20 +254,19 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
                 }
                 // table row of step s at o = 0 (ascending: p0 - 1 - s;
                 // descending: R0 - p0 + 1 + s); rows move by +-1 per o
-                uint32_t ta[KMAX];
+                const double2* ta[KMAX];
 #pragma unroll
-                for (int s = 0; s < KMAX; ++s)
-                    ta[s] = tabA_u + (uint32_t)((s * Mtab + (UB ? p0 - 1 - s : R0 - p0 + 1 + s)) * 16);
-                const uint32_t td = tabD_u + (uint32_t)((UB ? p0 - 1 - dstep : R0 - p0 + 1 + dstep) * 8);
+                for (int s = 0; s < KMAX; ++s) ta[s] = tabA + (s * Mtab + (UB ? p0 - 1 - s : R0 - p0 + 1 + s));
+                const double* td = tabD + (UB ? p0 - 1 - dstep : R0 - p0 + 1 + dstep);
 #pragma unroll
                 for (int o = 0; o < kSeqChunk; ++o) {
                     double v = vin[o];
 #pragma unroll
                     for (int s = 0; s < KMAX; ++s) {
                         if (s < K) {
-                            const double2 c = lds2(ta[s] + (UB ? 16 * o : -16 * o));
+                            const double2 c = ta[s][UB ? o : -o];
                             double y = xa[s];
-                            if (MV && s == dstep) y *= lds(td + (UB ? 8 * o : -8 * o));
+                            if (MV && s == dstep) y *= td[UB ? o : -o];
                             // z = (y - q z_prev) + o v: the part that does not
                             // depend on the step before is formed first, so
                             // the chain through the K steps is one FMA a step
@@ -298,9 +311,9 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
                     if (i < 0) {
                         z = 0.0;
                     } else if (i < Ms[s]) {
-                        const double2 c = lds2(tabA_u + (uint32_t)((s * Mtab + i) * 16));
+                        const double2 c = tabA[s * Mtab + i];
                         double y = xa[s];
-                        if (MV && s == dstep) y *= lds(tabD_u + (uint32_t)(i * 8));
+                        if (MV && s == dstep) y *= tabD[i];
                         if (SV) y = __fma_rn(-c.y, zp[s], y);
                         z = MV ? __fma_rn(c.x, v, y) : y;
                     } else {

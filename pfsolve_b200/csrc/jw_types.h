@@ -92,7 +92,7 @@ struct JwStepDesc {
     int64_t M;
     int64_t off_md, off_mo, off_sl, off_su;
     int diag;  // the matvec multiplies by the band diagonal (else by 1)
-    int pad;
+    unsigned perm_mul;  // reciprocal of perm_r (fast_div)
     int64_t perm_r, perm_m, perm_ceil, perm_floor;
 };
 
