@@ -42,7 +42,10 @@ struct DctShape {
     static constexpr int L8 = LOGN / 3;               // radix-8 stages
     static constexpr int REM = LOGN % 3;              // then one radix-2 (1) or radix-4 (2) stage
     static constexpr int NP = N + N / 8;  // the buffer, one 16-byte pad after every 8 values
-    static constexpr int NTW = N + N / 8 + N / 64 + 1;  // the twiddles, padded (dct_twpad)
+    // twiddles: a stage of radix R over Ns points reads k N/(Ns R), k < Ns, so
+    // none beyond N over the last stage's radix
+    static constexpr int NW = N / (REM == 0 ? 8 : (REM == 1 ? 2 : 4));
+    static constexpr int NTW = NW + NW / 8 + NW / 64 + 1;  // padded (dct_twpad)
     // one buffer of N complex values per row pair, then the twiddles
     static constexpr size_t SMEM = ((size_t)SPC * NP + NTW) * 16;
 };
@@ -117,16 +120,36 @@ __device__ __forceinline__ int dct_twpad(int i) { return i + (i >> 3) + (i >> 6)
 // One Stockham stage of radix R over N points with Ns points already
 // transformed per sub-sequence, in place: butterfly b reads buf[b + r N/R],
 // twiddles by e^{-2 pi i r k/(Ns R)} (k = b mod Ns), and, once every thread
-// of the row has read (`sync`), writes buf[(b - k) R + k + r Ns].  With
-// MAKHOUL_IN the buffer holds the rows in their natural order and the stage
-// reads sequence point p from Makhoul's position of it (2p for p < N/2,
-// 2N - 1 - 2p above); with OUT = 1 the stage writes point q there, so the
-// result leaves in the natural order.  Either way the reordering costs no
-// pass of its own, and both halves touch 8 different bank groups per access
+// of the row has read (`sync`), writes buf[(b - k) R + k + r Ns].  With OUT = 1
+// the stage writes point q to Makhoul's position of it (2q for q < N/2, 2N - 1
+// - 2q above), so the result leaves in the natural order: the reordering costs
+// no pass of its own, and both halves touch 8 different bank groups per access
 // phase.  OUT = 2 writes the natural order without the pads: type 2's last
 // stage, so that the post-processing's reads of Z_k and Z_{N-k} (ascending
 // and descending runs of 8) each touch 8 different bank groups.
-template <int R, int N, int TPS, bool MAKHOUL_IN = false, int OUT = 0, class SY>
+template <int N>
+__device__ __forceinline__ int dct_makhoul(int p)
+{
+    return p < N / 2 ? 2 * p : 2 * N - 1 - 2 * p;
+}
+template <int N, int OUT>
+__device__ __forceinline__ int dct_out_at(int q)
+{
+    if constexpr (OUT == 2) return q;
+    else return dct_pad(OUT == 1 ? dct_makhoul<N>(q) : q);
+}
+
+// The first stage (Ns = 1, no twiddles) on values a thread already holds:
+// a[r] is sequence point j + r N/8.
+template <int N, int OUT>
+__device__ __forceinline__ void dct_first_stage(double2* buf, int j, double2 (&a)[8])
+{
+    dct_dft<8>(a);
+#pragma unroll
+    for (int r = 0; r < 8; ++r) buf[dct_out_at<N, OUT>(8 * j + r)] = a[r];
+}
+
+template <int R, int N, int TPS, int OUT = 0, class SY>
 __device__ __forceinline__ void dct_stage(double2* buf, int Ns, int j, const double2* tw, SY sync)
 {
     constexpr int NBF = N / R, NB = NBF / TPS;
@@ -135,8 +158,7 @@ __device__ __forceinline__ void dct_stage(double2* buf, int Ns, int j, const dou
     for (int i = 0; i < NB; ++i)
 #pragma unroll
         for (int r = 0; r < R; ++r) {
-            const int p = j + i * TPS + r * NBF;
-            a[i][r] = buf[dct_pad(MAKHOUL_IN ? (p < N / 2 ? 2 * p : 2 * N - 1 - 2 * p) : p)];
+            a[i][r] = buf[dct_pad(j + i * TPS + r * NBF)];
         }
     sync();
 #pragma unroll
@@ -158,8 +180,7 @@ __device__ __forceinline__ void dct_stage(double2* buf, int Ns, int j, const dou
 #pragma unroll
         for (int r = 0; r < R; ++r) {
             const int q = base + r * Ns;
-            if constexpr (OUT == 2) buf[q] = a[i][r];
-            else buf[dct_pad(OUT == 1 ? (q < N / 2 ? 2 * q : 2 * N - 1 - 2 * q) : q)] = a[i][r];
+            buf[dct_out_at<N, OUT>(q)] = a[i][r];
         }
     }
     sync();
@@ -188,7 +209,7 @@ __global__ void __launch_bounds__(DctShape<LOGN>::NT, DctShape<LOGN>::NT <= 256 
     const int s = threadIdx.x / TPS, j = threadIdx.x - s * TPS;
     double2* buf = dct_smem + (size_t)s * S::NP;
     double2* tws = dct_smem + (size_t)S::SPC * S::NP;  // the twiddles, shared by the CTA's pairs
-    for (int i = threadIdx.x; i < N; i += blockDim.x) tws[dct_twpad(i)] = __ldg(&tw[i]);
+    for (int i = threadIdx.x; i < S::NW; i += blockDim.x) tws[dct_twpad(i)] = __ldg(&tw[i]);
     __syncthreads();
     // The threads of one pair synchronise among themselves only: a warp
     // (pairs of up to 256 points share warps, and keep in step), else a named
@@ -207,48 +228,46 @@ __global__ void __launch_bounds__(DctShape<LOGN>::NT, DctShape<LOGN>::NT <= 256 
         const double* x2 = io.in + io.in_off + (l2 ? y2 : 0) * io.in_stride;
 #pragma unroll
         for (int i = 0; i < PER; ++i) {
-            p1[i] = l1 ? x1[j + i * TPS] : 0.0;
-            p2[i] = l2 ? x2[j + i * TPS] : 0.0;
+            // what the first stage takes: sequence point j + i N/8 (type 2: at
+            // Makhoul's position, every second value of a run; its neighbours are
+            // another warp's, from L1)
+            const int p = TYPE == 2 ? dct_makhoul<N>(j + i * TPS) : j + i * TPS;
+            p1[i] = l1 ? x1[p] : 0.0;
+            p2[i] = l2 ? x2[p] : 0.0;
         }
     };
     int64_t u = (int64_t)blockIdx.x * S::SPC + s;
     fetch(u);
     for (int64_t base = (int64_t)blockIdx.x * S::SPC; base < npairs; base += stride_units, u += stride_units) {
-        if constexpr (TYPE == 2) {
-            // natural order; the first stage reads it in Makhoul's
-#pragma unroll
-            for (int i = 0; i < PER; ++i) buf[dct_pad(j + i * TPS)] = make_double2(p1[i], p2[i]);
-        } else {
-            // unpadded here, so that the descending reads of X_{N-k} touch 8
-            // different bank groups per access phase
-#pragma unroll
-            for (int i = 0; i < PER; ++i) buf[j + i * TPS] = make_double2(p1[i], p2[i]);
-            sync();
-            double2 Xr[PER];
-#pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                const int k = j + i * TPS;
-                Xr[i] = (k == 0) ? make_double2(0.0, 0.0) : buf[N - k];
-            }
-            sync();
-#pragma unroll
-            for (int i = 0; i < PER; ++i) {
-                const int k = j + i * TPS;
-                const double2 c = __ldg(&pt[k]);
-                // z_k = e^{-i t} (X_k + i X_{N-k}) = (X_k cos t + X_{N-k} sin t) + i (X_{N-k} cos t - X_k sin t)
-                const double z1r = __fma_rn(p1[i], c.x, Xr[i].x * c.y), z1i = __fma_rn(Xr[i].x, c.x, -(p1[i] * c.y));
-                const double z2r = __fma_rn(p2[i], c.x, Xr[i].y * c.y), z2i = __fma_rn(Xr[i].y, c.x, -(p2[i] * c.y));
-                buf[dct_pad(k)] = make_double2(z1r - z2i, z1i + z2r);  // z1 + i z2
-            }
-        }
-        sync();
-        fetch(u + stride_units);  // in flight while this pair is transformed
-        // The stages: the first reads type 2's rows in Makhoul's order, the
-        // last writes type 3's results in the rows' order and type 2's
-        // without the pads.
+        // The first stage works on registers: a thread holds the 8 points of its
+        // butterfly.  The last stage writes type 3's results in the rows' order
+        // and type 2's without the pads.
         constexpr int LAST = TYPE == 3 ? 1 : 2;
         constexpr int OUT8 = S::REM == 0 ? LAST : 0;  // the last radix-8 stage is the last
-        dct_stage<8, N, TPS, TYPE == 2, S::L8 == 1 ? OUT8 : 0>(buf, 1, j, tws, sync);
+        double2 a0[8];
+        if constexpr (TYPE == 2) {
+#pragma unroll
+            for (int i = 0; i < PER; ++i) a0[i] = make_double2(p1[i], p2[i]);
+        } else {
+            const int64_t y1 = 2 * u, y2 = 2 * u + 1;
+            const bool l1 = y1 < io.nsys, l2 = y2 < io.nsys;
+            const double* x1 = io.in + io.in_off + (l1 ? y1 : 0) * io.in_stride;
+            const double* x2 = io.in + io.in_off + (l2 ? y2 : 0) * io.in_stride;
+#pragma unroll
+            for (int i = 0; i < PER; ++i) {
+                const int k = j + i * TPS;
+                // X_{N-k}: loaded for another thread a moment ago (in L1)
+                const double r1 = (k > 0 && l1) ? x1[N - k] : 0.0, r2 = (k > 0 && l2) ? x2[N - k] : 0.0;
+                const double2 c = __ldg(&pt[k]);
+                // z_k = e^{-i t} (X_k + i X_{N-k}) = (X_k cos t + X_{N-k} sin t) + i (X_{N-k} cos t - X_k sin t)
+                const double z1r = __fma_rn(p1[i], c.x, r1 * c.y), z1i = __fma_rn(r1, c.x, -(p1[i] * c.y));
+                const double z2r = __fma_rn(p2[i], c.x, r2 * c.y), z2i = __fma_rn(r2, c.x, -(p2[i] * c.y));
+                a0[i] = make_double2(z1r - z2i, z1i + z2r);  // z1 + i z2
+            }
+        }
+        fetch(u + stride_units);  // in flight while this pair is transformed
+        dct_first_stage<N, S::L8 == 1 ? OUT8 : 0>(buf, j, a0);
+        sync();
         int Ns = 8;
 #pragma unroll 1
         for (int st = 1; st < S::L8 - 1; ++st) {
@@ -256,11 +275,11 @@ __global__ void __launch_bounds__(DctShape<LOGN>::NT, DctShape<LOGN>::NT <= 256 
             Ns *= 8;
         }
         if constexpr (S::L8 >= 2) {
-            dct_stage<8, N, TPS, false, OUT8>(buf, Ns, j, tws, sync);
+            dct_stage<8, N, TPS, OUT8>(buf, Ns, j, tws, sync);
             Ns *= 8;
         }
-        if constexpr (S::REM == 1) dct_stage<2, N, TPS, false, LAST>(buf, Ns, j, tws, sync);
-        else if constexpr (S::REM == 2) dct_stage<4, N, TPS, false, LAST>(buf, Ns, j, tws, sync);
+        if constexpr (S::REM == 1) dct_stage<2, N, TPS, LAST>(buf, Ns, j, tws, sync);
+        else if constexpr (S::REM == 2) dct_stage<4, N, TPS, LAST>(buf, Ns, j, tws, sync);
         const int64_t y1 = 2 * u, y2 = 2 * u + 1;
         const bool l1 = y1 < io.nsys, l2 = y2 < io.nsys;
         double* o1 = io.out + io.out_off + (l1 ? y1 : 0) * io.out_stride;
