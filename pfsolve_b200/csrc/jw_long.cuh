@@ -261,10 +261,16 @@ __device__ __forceinline__ void lg_solve(GroupCtx& g, const TB& coef, double Af,
     using BC = typename C::B;
     constexpr int R = C::R, U = BC::U;
     (void)R;
+    // A direction's band is read from the table once and stays in registers
+    // for the products after the scan (40 -> 24 bytes of table a row; shared
+    // memory bounds pass 2).
     if constexpr (BC::FWD) {
+        double2 nl[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) nl[u] = coef(BC::P_NL, u);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const double2 c = coef(BC::P_NL, u);
+            const double2 c = nl[u];
             if (u > 0) x[2 * u] = __fma_rn(c.x, x[2 * u - 1], x[2 * u]);
             x[2 * u + 1] = __fma_rn(c.y, x[2 * u], x[2 * u + 1]);
         }
@@ -275,7 +281,7 @@ __device__ __forceinline__ void lg_solve(GroupCtx& g, const TB& coef, double Af,
         double p = 1.0;
 #pragma unroll
         for (int u = 0; u < U; ++u) {
-            const double2 c = coef(BC::P_NL, u);
+            const double2 c = nl[u];
             p = c.x * p;
             x[2 * u] = __fma_rn(p, pin, x[2 * u]);
             p = c.y * p;
@@ -283,9 +289,12 @@ __device__ __forceinline__ void lg_solve(GroupCtx& g, const TB& coef, double Af,
         }
     }
     if constexpr (BC::BWD) {
+        double2 nh[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) nh[u] = coef(BC::P_NH, u);
 #pragma unroll
         for (int u = U - 1; u >= 0; --u) {
-            const double2 c = coef(BC::P_NH, u);
+            const double2 c = nh[u];
             if (u < U - 1) x[2 * u + 1] = __fma_rn(c.y, x[2 * u + 2], x[2 * u + 1]);
             x[2 * u] = __fma_rn(c.x, x[2 * u + 1], x[2 * u]);
         }
@@ -296,7 +305,7 @@ __device__ __forceinline__ void lg_solve(GroupCtx& g, const TB& coef, double Af,
         double p = 1.0;
 #pragma unroll
         for (int u = U - 1; u >= 0; --u) {
-            const double2 c = coef(BC::P_NH, u);
+            const double2 c = nh[u];
             p = c.y * p;
             x[2 * u + 1] = __fma_rn(p, q, x[2 * u + 1]);
             p = c.x * p;

@@ -630,6 +630,30 @@ struct StElem {
     __device__ __forceinline__ void finish() const { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 };
 
+// A solve band's chunk (-l or -h), read from the table once per system and kept
+// in registers for the products after the scan, where the chunk products have no
+// planes of their own and up to 16 rows per thread leave the registers; else
+// read again there.
+template <class C, class CT2>
+struct KeptBand {
+    static constexpr bool kKeep = !C::PRODS && C::R <= 16;
+    CT2 v[kKeep ? C::U : 1];
+    template <class F>
+    __device__ __forceinline__ KeptBand(const F& coef, int plane)
+    {
+        if constexpr (kKeep) {
+#pragma unroll
+            for (int u = 0; u < C::U; ++u) v[u] = coef(plane, u);
+        }
+    }
+    template <class F>
+    __device__ __forceinline__ CT2 operator()(const F& coef, int plane, int u) const
+    {
+        if constexpr (kKeep) return v[u];
+        else return coef(plane, u);
+    }
+};
+
 // ---- A group's systems sys, sys + step, ... < nsys, solved with the CTA's
 // coefficient table.  The first NBUF - 1 of them are being loaded into the
 // buffers from bi on; bi and par (the phase parity of bi's barrier) are left
@@ -997,9 +1021,10 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
         if constexpr (C::FWD && !C::MIXED && C::ALT) {
             // the same per system: z_j = x_j - l_j z_{j-2}; both systems' chunk
             // couplings in one paired scan
+            const KeptBand<C, CT2> nl(coef, C::P_NL);
 #pragma unroll
             for (int u = 1; u < U; ++u) {
-                const CT2 c = coef(C::P_NL, u);
+                const CT2 c = nl(coef, C::P_NL, u);
                 x[2 * u] = O::fma(c.x, x[2 * u - 2], x[2 * u]);
                 x[2 * u + 1] = O::fma(c.y, x[2 * u - 1], x[2 * u + 1]);
             }
@@ -1008,7 +1033,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
             CT p0 = 1, p1 = 1;
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const CT2 c = coef(C::P_NL, u);
+                const CT2 c = nl(coef, C::P_NL, u);
                 p0 = c.x * p0;
                 x[2 * u] = O::fma(p0, pin0, x[2 * u]);
                 p1 = c.y * p1;
@@ -1040,9 +1065,10 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
         if constexpr (C::FWD && !C::MIXED && !C::ALT && !C::QUAD) {
             // z_j = x_j - l_j z_{j-1} within the chunk, then add the coupling
             // from the preceding chunks scaled by prod_{k<=j}(-l_k)
+            const KeptBand<C, CT2> nl(coef, C::P_NL);
 #pragma unroll
             for (int u = 0; u < U; ++u) {
-                const CT2 c = coef(C::P_NL, u);
+                const CT2 c = nl(coef, C::P_NL, u);
                 if (u > 0) x[2 * u] = O::fma(c.x, x[2 * u - 1], x[2 * u]);
                 x[2 * u + 1] = O::fma(c.y, x[2 * u], x[2 * u + 1]);
             }
@@ -1060,7 +1086,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
                 CT p = 1;
 #pragma unroll
                 for (int u = 0; u < U; ++u) {
-                    const CT2 c = coef(C::P_NL, u);
+                    const CT2 c = nl(coef, C::P_NL, u);
                     p = c.x * p;
                     x[2 * u] = O::fma(p, pin, x[2 * u]);
                     p = c.y * p;
@@ -1069,9 +1095,10 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
             }
         }
         if constexpr (C::BWD && !C::MIXED && C::ALT) {
+            const KeptBand<C, CT2> nh(coef, C::P_NH);
 #pragma unroll
             for (int u = U - 2; u >= 0; --u) {
-                const CT2 c = coef(C::P_NH, u);
+                const CT2 c = nh(coef, C::P_NH, u);
                 x[2 * u + 1] = O::fma(c.y, x[2 * u + 3], x[2 * u + 1]);
                 x[2 * u] = O::fma(c.x, x[2 * u + 2], x[2 * u]);
             }
@@ -1080,7 +1107,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
             CT p0 = 1, p1 = 1;
 #pragma unroll
             for (int u = U - 1; u >= 0; --u) {
-                const CT2 c = coef(C::P_NH, u);
+                const CT2 c = nh(coef, C::P_NH, u);
                 p1 = c.y * p1;
                 x[2 * u + 1] = O::fma(p1, q1, x[2 * u + 1]);
                 p0 = c.x * p0;
@@ -1108,9 +1135,10 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
             }
         }
         if constexpr (C::BWD && !C::MIXED && !C::ALT && !C::QUAD) {
+            const KeptBand<C, CT2> nh(coef, C::P_NH);
 #pragma unroll
             for (int u = U - 1; u >= 0; --u) {
-                const CT2 c = coef(C::P_NH, u);
+                const CT2 c = nh(coef, C::P_NH, u);
                 if (u < U - 1) x[2 * u + 1] = O::fma(c.y, x[2 * u + 2], x[2 * u + 1]);
                 x[2 * u] = O::fma(c.x, x[2 * u + 1], x[2 * u]);
             }
@@ -1128,7 +1156,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
                 CT p = 1;
 #pragma unroll
                 for (int u = U - 1; u >= 0; --u) {
-                    const CT2 c = coef(C::P_NH, u);
+                    const CT2 c = nh(coef, C::P_NH, u);
                     p = c.y * p;
                     x[2 * u + 1] = O::fma(p, q, x[2 * u + 1]);
                     p = c.x * p;
