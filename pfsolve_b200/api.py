@@ -64,6 +64,7 @@ class App:
         if outputBuffer is not None:
             cfg.outputBuffer = self._vpp(outputBuffer)
         self.app = capi.PfSolveApplication()
+        self._app_p = ctypes.pointer(self.app)
         check(self._lib.initializePfSolve(ctypes.byref(self.app), cfg), "initializePfSolve")
         self.alive = True
 
@@ -137,12 +138,16 @@ def device_status() -> int:
     return int(capi.load().PfSolveGetDeviceStatus())
 
 
+_AppPtr = ctypes.POINTER(capi.PfSolveApplication)
+_LaunchPtr = ctypes.POINTER(capi.PfSolveLaunchParams)
+
+
 def append_chain(apps: Sequence[App], lps: Sequence[capi.PfSolveLaunchParams], allow_unfused: bool = False):
     """Run apps as one fused kernel (``PfSolveAppendChain``)."""
     lib = capi.load()
     n = len(apps)
-    app_ptrs = (ctypes.POINTER(capi.PfSolveApplication) * n)(*[ctypes.pointer(a.app) for a in apps])
-    lp_ptrs = (ctypes.POINTER(capi.PfSolveLaunchParams) * n)(*[ctypes.pointer(l) for l in lps])
+    app_ptrs = (_AppPtr * n)(*[a._app_p for a in apps])
+    lp_ptrs = (_LaunchPtr * n)(*map(ctypes.pointer, lps))
     check(lib.PfSolveAppendChain(app_ptrs, lp_ptrs, n, 1 if allow_unfused else 0), "PfSolveAppendChain")
 
 
