@@ -58,6 +58,11 @@ struct AppState {
         const StreamVariant* v = nullptr;
         int G = 0, max_blocks = 0, nbuf = 2;
     } stream_pair, elem_pair;
+    // double-double: the forms for many and for few systems (choose_dd)
+    struct Form {
+        const JwVariant* v = nullptr;
+        int W = 1, G = 1, max_blocks = 0;
+    } dd_many, dd_few;
     int stream_G = 0, stream_max_blocks = 0;
     int stream_nbuf = 2;  // staging buffers per group
     int nbuf_req = 0;     // caller's staging buffers per group (0: choose)
@@ -106,6 +111,7 @@ struct AppState {
         const StreamVariant* elem_v;
         int elem_G, elem_max_blocks, elem_nbuf;
         Pair stream_pair, elem_pair;
+        Form dd_many, dd_few;
     };
     std::vector<ChainPlan> chain_plans;
     // streams
@@ -542,6 +548,29 @@ PfSolveResult plan_alt(AppState* s, const PfSolveConfiguration& c, int base_prec
 // Pick the kernel variant and launch shape for M rows: register variants
 // first, then coefficient-table variants (FP64); rows per thread from the
 // caller's choice (s->R) first, then the other compiled choices.
+// Double-double launches of a table-form plan whose rows per thread the caller
+// left open.  Many systems: the table form with the shortest capacity that
+// holds M rows -- 4, 8 and 16 rows per thread of one warp, 16 of two (2^23
+// rows: N = 33 1 361 us at 16 rows of one warp, 461 at 4; 128 383 and 133;
+// 256 205 and 115 at 8; 700 254 at 8 rows of four warps, 182 at 16 of two;
+// 1 000 174 and 140).  Up to three rounds of its resident groups: the register
+// form at 4 rows per thread, whose prologue and solve are the shortest (8
+// systems: N = 512 13.5 against 22.8 us, 1 000 17.7 against 24).
+void choose_dd(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
+{
+    auto take = [&](int R, int tbl, AppState::Form& f) {
+        const int64_t W = (M + 32 * (int64_t)R - 1) / (32 * (int64_t)R);
+        const JwVariant* v = find_jw_variant(R, s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, tbl);
+        if (!v || W > 8 || 32 * W > v->max_threads || !choose_groups(v, (int)W, s->num_sms, f.G, f.max_blocks)) return;
+        f.v = v;
+        f.W = (int)W;
+    };
+    if (M > 1024) return;
+    take(M <= 128 ? 4 : (M <= 256 ? 8 : 16), 1, s->dd_many);
+    take(4, 0, s->dd_few);
+    cudaGetLastError();
+}
+
 PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
 {
     // Double-double: the table form first (16 rows per thread where a system
@@ -552,7 +581,8 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
         const int cand[3][2] = {{16, 1}, {8, 1}, {4, 1}};
         for (const auto& rc : cand) {
             const int R = rc[0];
-            if (s->R_req && R != s->R_req) continue;
+            // (a caller's 4: the register form)
+            if (s->R_req && (R != s->R_req || R == 4)) continue;
             const int64_t W = (M + 32 * (int64_t)R - 1) / (32 * (int64_t)R);
             if (W < 1 || W > 4 || (R == 16 && W > 1 && !s->R_req)) continue;
             const JwVariant* v = find_jw_variant(R, s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, 1);
@@ -564,6 +594,7 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
             s->W = (int)W;
             s->G = G;
             s->max_blocks = maxb;
+            if (!s->R_req) choose_dd(s, M, LIN, LOUT, SCALE);
             return PFSOLVE_SUCCESS;
         }
     }
@@ -870,16 +901,23 @@ PfSolveResult launch_jw_variant(AppState* s, const JwOperator& op, const JwIO& i
         return PFSOLVE_SUCCESS;
     }
     if (!s->variant) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;  // streaming-only plan
-    const int64_t want = (io.nsys + s->G - 1) / s->G;
-    int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, s->max_blocks));
+    AppState::Form f;
+    f.v = s->variant;
+    f.W = s->W;
+    f.G = s->G;
+    f.max_blocks = s->max_blocks;
+    if (s->dd_few.v && io.nsys <= 3 * (int64_t)s->dd_few.max_blocks * s->dd_few.G) f = s->dd_few;
+    else if (s->dd_many.v) f = s->dd_many;
+    const int64_t want = (io.nsys + f.G - 1) / f.G;
+    int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, f.max_blocks));
     // ALT: a group keeps one parity, so the system step (grid x groups) is even
-    if (io.alt && (grid * s->G) % 2) grid = grid > 1 ? grid - 1 : 2;
-    const size_t smem = s->variant->smem_bytes(s->W, s->G);
-    s->variant->launch(dim3((unsigned)grid), dim3(32 * s->W * s->G), smem, stream, op, io, s->W);
+    if (io.alt && (grid * f.G) % 2) grid = grid > 1 ? grid - 1 : 2;
+    const size_t smem = f.v->smem_bytes(f.W, f.G);
+    f.v->launch(dim3((unsigned)grid), dim3(32 * f.W * f.G), smem, stream, op, io, f.W);
     g_launches.fetch_add(1, std::memory_order_relaxed);
     {
-        const JwVariant* v = s->variant;
-        record_launch(PFSOLVE_KERNEL_GROUP, v->R, s->W, s->G, v->KL, v->KU, v->SV, v->LIN, v->LOUT, v->SCALE, v->PREC,
+        const JwVariant* v = f.v;
+        record_launch(PFSOLVE_KERNEL_GROUP, v->R, f.W, f.G, v->KL, v->KU, v->SV, v->LIN, v->LOUT, v->SCALE, v->PREC,
                       io.alt, grid);
     }
     if (cudaPeekAtLastError() != cudaSuccess) {
@@ -1678,6 +1716,8 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
         t.elem_nbuf = cp.elem_nbuf;
         t.stream_pair = cp.stream_pair;
         t.elem_pair = cp.elem_pair;
+        t.dd_many = cp.dd_many;
+        t.dd_few = cp.dd_few;
         return launch_jw_variant(&t, op, io, stream);
     }
     AppState t;
@@ -1698,7 +1738,8 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
     sj->chain_plans.push_back(AppState::ChainPlan{KL, KU, L.sv, LIN, LOUT, SCALE, t.variant, t.R, t.W, t.G,
                                                   t.max_blocks, t.stream_v, t.stream_G, t.stream_max_blocks,
                                                   t.stream_nbuf, t.elem_v, t.elem_G, t.elem_max_blocks,
-                                                  t.elem_nbuf, t.stream_pair, t.elem_pair});
+                                                  t.elem_nbuf, t.stream_pair, t.elem_pair, t.dd_many,
+                                                  t.dd_few});
     return launch_jw_variant(&t, op, io, stream);
 }
 

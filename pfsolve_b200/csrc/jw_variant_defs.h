@@ -60,7 +60,8 @@ inline void dd_tbl_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st
 #define PFB_DD(KL, KU, SV)                                                                                 \
     PFB_DDV(4, KL, KU, SV, true), PFB_DDV(8, KL, KU, SV, true), PFB_DDV(4, KL, KU, SV, false),               \
         PFB_DDV(8, KL, KU, SV, false), PFB_DDT(8, KL, KU, SV, true), PFB_DDT(16, KL, KU, SV, true),          \
-        PFB_DDT(8, KL, KU, SV, false), PFB_DDT(16, KL, KU, SV, false)
+        PFB_DDT(8, KL, KU, SV, false), PFB_DDT(16, KL, KU, SV, false),                                       \
+        PFB_DDT(4, KL, KU, SV, true), PFB_DDT(4, KL, KU, SV, false)
 
 // Rows-per-thread choices for the single-application (drop-in) variants.
 #define PFB_R4(KL, KU, SV, LIN, LOUT, SC) \
