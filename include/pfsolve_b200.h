@@ -368,8 +368,10 @@ PFSOLVE_API PfSolveResult PfSolveAppendChain(PfSolveApplication** apps, PfSolveL
  * the chain [dgbmv] -> JW -> [block] of the apps with the same fields.
  * Every entry uses plan-time band offsets: JW bands at 0, M, 2M of `bands`
  * (reference register-major order for its own M), dgbmv bands band-major.
- * Two kernels: the group kernel (a group of warps per system, rowsPerThread
- * rows per thread) and the sweep kernel (one complex system per lane, its
+ * Three kernels: the group kernel (a group of warps per system, rowsPerThread
+ * rows per thread), the streaming solve for real systems (a CTA per item, its
+ * table built once; the default for real systems of at most 2048 rows without
+ * accumulation) and the sweep kernel (one complex system per lane, its
  * rows in sequence, a warp per item of 32 systems).  sweepRows = 8 or 16
  * asks for the sweep kernel with that many rows per staged chunk
  * (PFSOLVE_ERROR_UNSUPPORTED_COMBINATION where the batch does not allow it).
@@ -417,13 +419,16 @@ PFSOLVE_API PfSolveResult PfSolveBatchAppend(PfSolveBatch* batch, cudaStream_t s
  * stream); later PfSolveBatchAppend calls launch the graph. */
 PFSOLVE_API PfSolveResult PfSolveBatchCaptureGraph(PfSolveBatch* batch, cudaStream_t stream);
 /* Time every compiled rows-per-thread / item-size candidate of the group
- * kernel, and the sweep kernel where the batch allows it, on the batch's own
+ * kernel, and the sweep kernel and the streaming solve where the batch allows
+ * them, on the batch's own
  * buffers (`iterations` launches each) and keep the fastest; drops a
  * captured graph.  Entries must be out of place (input != output). */
 PFSOLVE_API PfSolveResult PfSolveBatchAutotune(PfSolveBatch* batch, cudaStream_t stream, int iterations);
 /* Chosen shape: rows per thread, warps per system, systems per item, work
  * items, and the autotuner's best time (ms, 0 when not tuned).  Rows per
- * thread and warps per system 0: the sweep kernel. */
+ * thread and warps per system 0: the sweep kernel.  On the streaming solve the
+ * shape is that of the longest entry and the item size that of the largest
+ * item (each entry has its own). */
 PFSOLVE_API PfSolveResult PfSolveBatchGetShape(const PfSolveBatch* batch, int* rowsPerThread, int* warpsPerSystem,
                                                int* systemsPerItem, int* items, double* tunedMs);
 /* The sweep kernel's shape: rows per staged chunk, chunk buffers per warp and
@@ -477,8 +482,12 @@ PFSOLVE_API PfSolveResult PfSolveGetDeviceStatus(void);
 
 /* Kernel shape a JW or dgbmv plan chose: streaming = 1 when its launches use
  * the TMA-staged streaming kernel wherever their buffers allow it, with
- * rowsPerThread x warpsPerSystem rows per group and groupsPerCTA groups;
- * streaming = 0: the group kernel's shape; streaming = 2: long systems
+ * rowsPerThread x warpsPerSystem rows per group and groupsPerCTA groups
+ * (large batches of real systems run it with fewer groups that solve two
+ * systems each);
+ * streaming = 0: the group kernel's shape (its larger launches take the
+ * streaming kernel with element copies, and double-double launches a form
+ * chosen by their number of systems: PfSolveGetLastLaunch); streaming = 2: long systems
  * (M > 4096), one thread-block cluster per system, warpsPerSystem warps over
  * the cluster's CTAs; streaming = 3: the K-step kernel
  * (numConsecutiveJWIterations > 1); streaming = 4: K bidiagonal steps with one

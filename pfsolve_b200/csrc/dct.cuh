@@ -19,11 +19,15 @@
 // radix-8 butterfly per stage (N/8 threads per row), and a CTA holds as many
 // row pairs as 256 threads cover: one FFT transforms two rows (see the
 // kernel).  Each thread loads the next pair's inputs into registers while the
-// current pair is transformed.  Twiddles e^{-2 pi i j/N} and the
+// current pair is transformed: the eight points of its first butterfly, so the
+// first stage starts from registers and the rows are not staged before it.
+// (Types 2 and 3 together over 2^25 points, with and without that staging: N =
+// 64 217 and 201 us, 512 232 and 216, 2 048 313 and 289, 4 096 355 and 340.
+// Three or four CTAs an SM at 85 or 64 registers, without the prefetch, were
+// slower: the shared-memory and FP64 issue slots bound the kernel.)  Twiddles e^{-2 pi i j/N} and the
 // pre/post factors (cos, sin)(pi k/2N) come from tables the plan computes once
-// in long double on the host.  Rows are read and written with coalesced
-// global accesses; a row is fully staged before its result is written, so
-// the transform may run in place.  The step is bound by HBM bandwidth at
+// in long double on the host.  A row is fully read before its result is
+// written, so the transform may run in place.  The step is bound by HBM bandwidth at
 // large batches (16 bytes moved per point, in and out).
 #pragma once
 #include <cstdint>
@@ -198,7 +202,8 @@ __device__ __forceinline__ void dct_stage(double2* buf, int Ns, int j, const dou
 //           Re FFT(c) = FFT(z1) and Im FFT(c) = FFT(z2).
 // One buffer of N complex values per pair; each thread keeps the next pair's
 // 2 N/TPS input values in registers, loaded while the current pair is
-// transformed.
+// transformed; type 3 reads X_{N-k} when the pair's turn comes, from L1 (as
+// X_k it was another thread's a moment ago).
 template <int LOGN, int TYPE>
 __global__ void __launch_bounds__(DctShape<LOGN>::NT, DctShape<LOGN>::NT <= 256 ? 2 : 1)
     dct_kernel(const DctIO io, const double2* __restrict__ tw, const double2* __restrict__ pt)

@@ -633,7 +633,8 @@ struct StElem {
 // A solve band's chunk (-l or -h), read from the table once per system and kept
 // in registers for the products after the scan, where the chunk products have no
 // planes of their own and up to 16 rows per thread leave the registers; else
-// read again there.
+// read again there.  (32 768 ALT row sets of 1 024 rows 119 -> 103 us, 8 192 of
+// 4 096 216 -> 169; FP64 on FP32 storage, 47 866 x 701: 158 -> 134.)
 template <class C, class CT2>
 struct KeptBand {
     static constexpr bool kKeep = !C::PRODS && C::R <= 16;
