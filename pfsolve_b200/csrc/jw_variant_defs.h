@@ -39,7 +39,7 @@ template <class C>
 inline void dd_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const JwOperator& op, const JwIO& io,
                          int W)
 {
-    jw_dd_kernel<C><<<grid, block, smem, st>>>(op, io, W);
+    jw_dd_kernel<C><<<grid, block, smem, st>>>(op, dd_io(io), W);
 }
 #define PFB_DDV(R, KL, KU, SV, MEM)                                                                     \
     JwVariant{R, KL, KU, SV, LAY_REAL, LAY_REAL, 0, (MEM) ? 2 : 3, 0, 256,                              \
@@ -49,7 +49,7 @@ template <class C>
 inline void dd_tbl_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const JwOperator& op,
                              const JwIO& io, int W)
 {
-    jw_dd_tbl_kernel<C><<<grid, block, smem, st>>>(op, io, W);
+    jw_dd_tbl_kernel<C><<<grid, block, smem, st>>>(op, dd_io(io), W);
 }
 // table form (TBL = 1): coefficients, chunk products and scan multipliers in
 // shared memory
