@@ -706,6 +706,7 @@ void fill_operator_common(AppState* s, const PfSolveConfiguration& c, JwOperator
 struct MapCacheEntry {
     const void* v;  // the stream or cluster variant the maps were encoded for
     JwIO io;
+    int64_t sets;  // StreamIO::sets
     CUtensorMap in, out;
     bool valid;
 };
@@ -715,25 +716,27 @@ thread_local unsigned g_map_next = 0;
 bool same_io(const JwIO& a, const JwIO& b)
 {
     return a.in == b.in && a.out == b.out && a.in_off == b.in_off && a.in_stride == b.in_stride &&
-           a.out_off == b.out_off && a.out_stride == b.out_stride && a.nsys == b.nsys && a.M == b.M && a.sets == b.sets;
+           a.out_off == b.out_off && a.out_stride == b.out_stride && a.nsys == b.nsys && a.M == b.M;
 }
 
-const MapCacheEntry* row_maps(const void* key, int R, int LIN, int LOUT, int IB, int IBO, const JwIO& io, int es = 8)
+const MapCacheEntry* row_maps(const void* key, int R, int LIN, int LOUT, int IB, int IBO, const JwIO& io, int es = 8,
+                              int64_t sets = 0)
 {
     for (const MapCacheEntry& e : g_map_cache)
-        if (e.valid && e.v == key && same_io(e.io, io)) return &e;
+        if (e.valid && e.v == key && e.sets == sets && same_io(e.io, io)) return &e;
     MapCacheEntry& e = g_map_cache[g_map_next++ % 8];
     e.valid = false;
-    if (!encode_row_maps(R, LIN, LOUT, IB, IBO, io, &e.in, &e.out, es)) return nullptr;
+    if (!encode_row_maps(R, LIN, LOUT, IB, IBO, io, &e.in, &e.out, es, sets)) return nullptr;
     e.v = key;
     e.io = io;
+    e.sets = sets;
     e.valid = true;
     return &e;
 }
 
-const MapCacheEntry* stream_maps(const StreamVariant* v, const JwIO& io)
+const MapCacheEntry* stream_maps(const StreamVariant* v, const StreamIO& io)
 {
-    return row_maps(v, v->R, v->LIN, v->LOUT, v->IB, v->IBO, io, prec_f32_storage(v->PREC) ? 4 : 8);
+    return row_maps(v, v->R, v->LIN, v->LOUT, v->IB, v->IBO, io, prec_f32_storage(v->PREC) ? 4 : 8, io.sets);
 }
 
 // Long systems: the cluster kernel, under the streaming kernel's buffer rules.
@@ -804,7 +807,7 @@ PfSolveResult launch_long(AppState* s, const JwOperator& op, const JwIO& io, cud
 // that every table value read from shared memory (the streaming kernel's bound
 // on real systems) serves two.  Worth it once every resident pair has two
 // rounds of work.
-bool take_pairs(const AppState::Pair& p, JwIO& io)
+bool take_pairs(const AppState::Pair& p, StreamIO& io)
 {
     if (!p.v || io.nsys < 4 * (int64_t)p.max_blocks * p.G) return false;
     io.sets = io.nsys;
@@ -820,7 +823,7 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
     const StreamVariant* v = s->stream_v;
     if (!v || io.accumulate || io.oz0 > 0 || io.oz1 < io.M) return false;
     // ALT: the launch counts systems (two per row set); the kernel, row sets
-    JwIO rs = io;
+    StreamIO rs(io);
     if (v->ALT) rs.nsys = io.nsys / 2;
     int G = s->stream_G, max_blocks = s->stream_max_blocks;
     rs.nbuf = s->stream_nbuf;
@@ -857,7 +860,7 @@ bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t
     const uintptr_t in0 = reinterpret_cast<uintptr_t>(io.in) + (uintptr_t)io.in_off * es;
     const uintptr_t out0 = reinterpret_cast<uintptr_t>(io.out) + (uintptr_t)io.out_off * es * (packed ? 2 : 1);
     if (in0 % es || out0 % (packed ? 2 * es : es)) return false;
-    JwIO eio = io;
+    StreamIO eio(io);
     if (v->ALT) eio.nsys = io.nsys / 2;  // row sets, two systems each
     eio.nbuf = s->elem_nbuf;
     eio.unit16 = in0 % 16 == 0 && (io.in_stride * es) % 16 == 0 &&
@@ -1010,10 +1013,8 @@ PfSolveResult append_steps(PfSolveApplication* app, const PfSolveLaunchParams* l
         const int64_t grid = std::min<int64_t>(s->num_sms, (nblk + nw - 1) / nw);
         const int64_t Mtab = c.upperBanded ? S.M_in : S.M_out;
         // few sweeping warps: more that only help to build the step tables
-        io.groups = nw;
-        s->seq_v->launch(dim3((unsigned)grid), dim3(32 * std::max(nw, 12)), seq_steps_smem_bytes(S.K, Mtab, nw, s->seq_v->CH), stream,
-                         &tin, &tout,
-                         S, io);
+        s->seq_v->launch(dim3((unsigned)grid), dim3(32 * std::max(nw, 12)),
+                         seq_steps_smem_bytes(S.K, Mtab, nw, s->seq_v->CH), stream, &tin, &tout, S, io, nw);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         record_launch(PFSOLVE_KERNEL_STEPS_SWEEP, 0, 0, nw, c.upperBanded == 0 ? 1 : 0, c.upperBanded == 1 ? 1 : 0,
                       s->seq_v->SV ? (c.upperBanded ? SV_LOWER : SV_UPPER) : SV_NONE, LAY_REAL, LAY_REAL, 0,

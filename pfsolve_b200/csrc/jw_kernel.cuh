@@ -627,9 +627,13 @@ __device__ __forceinline__ void issue_segment_load(const JwIO& io, int64_t sys, 
 {
     using T = typename C::T;
     constexpr int R = C::kR, KL = C::kKL, KU = C::kKU;
-    const int64_t M = io.M;
+    const int M = (int)io.M;
     const T* in = reinterpret_cast<const T*>(io.in);
-    auto row_ok = [&](int64_t row) { return row >= 0 && row < M && row >= io.iz0 && row < io.iz1; };
+    // rows read: [lo, hi), in 32 bits (four 64-bit comparisons a row cost the
+    // FP64 bidiagonal kinds 8 %: 65 536 x 512 173.6 -> 158.9 us, ALT 131 072 x
+    // 1 024 854 -> 781)
+    const int lo = (int)max((int64_t)0, min(io.iz0, io.M)), hi = (int)max((int64_t)0, min(io.iz1, io.M));
+    auto row_ok = [&](int64_t row) { return (int)row >= lo && (int)row < hi; };
     if constexpr (C::kLIN == LAY_REAL) {
         // ALT: row e of system sys is row 2 e + (sys & 1) of row set sys / 2
         const int64_t h = io.alt ? (sys & 1) : 0, es = io.alt ? 2 : 1;
@@ -680,14 +684,23 @@ __device__ __forceinline__ void store_segment(const JwIO& io, int64_t sys, int64
     using T2 = typename Vec2Of<T>::type;
     constexpr int R = C::kR;
     T* out = reinterpret_cast<T*>(io.out);
+    // Row arithmetic in 32 bits for the mixed mode only: there it takes 65 536 x
+    // 512 from 488 to 466 us (tridiagonal) and 343 to 328 (bidiagonal, band above);
+    // FP64 tridiagonal kinds of eight warps lose with it (30 000 x 1 001 195 -> 290).
+    using I = typename std::conditional<C::kMixed, int, int64_t>::type;
     const int64_t M = io.M;
-    const int64_t h = io.alt ? (sys & 1) : 0, es = io.alt ? 2 : 1;
-    const int64_t Msys = io.alt ? (M - h + 1) >> 1 : M;
+    const I h = io.alt ? (I)(sys & 1) : 0, es = io.alt ? 2 : 1;
+    const I Msys = (I)(io.alt ? (M - h + 1) >> 1 : M);
+    const I lo = (I)max((int64_t)0, min(io.oz0, M)), hi = (I)max((int64_t)0, min(io.oz1, M));
 #pragma unroll
     for (int k = 0; k < R; ++k) {
         const int q = 32 * k + lane;
-        const int64_t row = r0 + q;
-        if (row >= Msys || es * row + h < io.oz0 || es * row + h >= io.oz1) continue;
+        const I row = (I)r0 + q;
+        if constexpr (C::kMixed) {
+            if (es * row + h < lo || es * row + h >= hi) continue;
+        } else {
+            if (row >= Msys || es * row + h < io.oz0 || es * row + h >= io.oz1) continue;
+        }
         if constexpr (C::kLOUT == LAY_REAL) {
             T v = buf[swz<R, false>(q)];
             T* p = out + io.out_off + (io.alt ? sys >> 1 : sys) * io.out_stride + es * row + h;
@@ -925,8 +938,14 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_step_kernel(const JwOperato
 // (largest items first), refactors when the entry changes and streams the
 // item's systems.  Item fetch: the group leader's atomicAdd is broadcast
 // through two alternating shared slots, one barrier per fetch.
+// Two CTAs an SM where the coefficients and the data fit 128 registers with hardly
+// a spill: 4 rows per thread, and 8 of a one-band, one-sided FP64 solve (1 500
+// entries of one 2 000-row system: 93.8 us with two, 104.8 with one at 223).
 template <class C>
-__global__ void __launch_bounds__(256) jw_batch_kernel(const BatchEntryDev* __restrict__ entries,
+constexpr int kBatchCtas =
+    (C::kR <= 4 || (C::kR <= 8 && C::NB == 1 && C::kSV != SV_TRI && !C::kMixed && !C::kCplx)) ? 2 : 1;
+template <class C>
+__global__ void __launch_bounds__(256, kBatchCtas<C>) jw_batch_kernel(const BatchEntryDev* __restrict__ entries,
                                                       const WorkItem* __restrict__ items, const int nitems,
                                                       unsigned int* __restrict__ counter, const int W)
 {

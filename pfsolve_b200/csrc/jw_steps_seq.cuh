@@ -75,7 +75,8 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
 template <int UB, bool MV, bool SV, int K, int CH>
 __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                                       const __grid_constant__ CUtensorMap tm_out,
-                                                                      const __grid_constant__ JwSteps S, const JwIO io)
+                                                                      const __grid_constant__ JwSteps S, const JwIO io,
+                                                                      const int NW)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int kSeqChunk = CH, kSeqBufBytes = seq_buf_bytes(CH), kSeqBufs = seq_nbufs(K, CH);
@@ -83,7 +84,7 @@ __global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(cons
     constexpr int CS = CH == 16 ? 4 : 3;        // chunk of a sweep position: >> CS
     constexpr int ROWB = CH * 8;                // bytes of a system's row in a box
     constexpr int KMAX = K;
-    const int NW = io.groups;  // sweeping warps; any others only help with the table
+    // NW sweeping warps; any others only help with the table
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int M0 = (int)S.M_in, Mout = (int)S.M_out;
     const int Mtab = UB ? M0 : Mout;  // rows of the widest step

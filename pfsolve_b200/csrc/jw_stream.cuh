@@ -531,7 +531,7 @@ template <class C>
 struct StElem {
     static constexpr int kArrivals = C::T;
     using Sto = typename C::Sto;
-    const JwIO* io;
+    const StreamIO* io;
     unsigned char* base;
     uint64_t* bars;
     int wg, lane;
@@ -1231,7 +1231,7 @@ __device__ __forceinline__ bool st_run(const JwOperator& op, const JwIO& io, con
 // ---- The kernels: one CTA per SM, G groups, a table, every group its share of
 // the systems.
 template <class C, class LD>
-__device__ __forceinline__ void st_kernel(const JwOperator& op, const JwIO& io, LD ld)
+__device__ __forceinline__ void st_kernel(const JwOperator& op, const StreamIO& io, LD ld)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using CT = typename C::CT;
@@ -1283,7 +1283,7 @@ __device__ __forceinline__ void st_kernel(const JwOperator& op, const JwIO& io, 
 template <class C>
 __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                                   const __grid_constant__ CUtensorMap tm_out,
-                                                                  const JwOperator op, const JwIO io)
+                                                                  const JwOperator op, const StreamIO io)
 {
     StTma<C> ld;
     ld.tm_in = &tm_in;
@@ -1295,7 +1295,7 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_
 // that R does not divide.
 template <class C>
 __global__ void __launch_bounds__(C::kMaxThreads) jw_stream_elem_kernel(const JwOperator op,
-                                                                       const __grid_constant__ JwIO io)
+                                                                       const __grid_constant__ StreamIO io)
 {
     StElem<C> ld;
     ld.io = &io;

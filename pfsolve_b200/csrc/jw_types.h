@@ -76,9 +76,21 @@ struct JwIO {
     int alt;                      // ALT mode: system 2y + h is the parity-h rows of row set y
     int plain;                    // long-system single pass: rows not 16-byte aligned, moved by plain loads/stores
     int nbuf;                     // streaming kernel: staging buffers per group (2..4; 0: 2)
-    int groups;                   // streaming kernel: groups per CTA
-    int64_t sets;                 // real systems solved in pairs as XXII ones: their number (0: 2 nsys row sets)
-    int unit16;                   // streaming kernel, element copies: rows, strides and bases in whole 16-byte units
+};
+// Every other kernel takes a JwIO by value.  A struct argument of up to 128
+// bytes is held in registers, a larger one is read from parameter memory at
+// each use: with 24 bytes more the group kernel's main loop lost up to a fifth
+// (ALT, 131 072 row sets of 1 024 rows, 875 -> 1 022 us; 65 536 x 512
+// tridiagonal 221 -> 263).
+static_assert(sizeof(JwIO) <= 128, "kernel argument held in registers");
+
+// The streaming kernels' data side.
+struct StreamIO : JwIO {
+    int groups;    // groups per CTA
+    int64_t sets;  // real systems solved in pairs as XXII ones: their number (0: 2 nsys row sets)
+    int unit16;    // element copies: rows, strides and bases in whole 16-byte units
+    StreamIO() = default;
+    explicit StreamIO(const JwIO& io) : JwIO(io), groups(0), sets(0), unit16(0) {}
 };
 
 // K consecutive steps in one kernel (numConsecutiveJWIterations = K).
@@ -109,7 +121,7 @@ struct JwSteps {
 // a work list of (entry, system range) items consumed through a counter.
 struct BatchEntryDev {
     JwOperator op;
-    JwIO io;
+    StreamIO io;
 };
 struct WorkItem {
     int entry;

@@ -88,7 +88,7 @@ struct StreamVariant {
     size_t (*smem_bytes)(int G, int NB);  // G groups of NB staging buffers
     int IB, IBO;
     void (*launch)(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const CUtensorMap* in, const CUtensorMap* out,
-                   const JwOperator& op, const JwIO& io);
+                   const JwOperator& op, const StreamIO& io);
     int ALT = 0;  // ALT stride-2 mode: one staged row set holds two systems (its even and odd rows)
     int (*threads)(int G) = nullptr;  // threads of a CTA of G groups
     int ELEM = 0; // systems staged by element copies (any row count, stride and offset); `in`, `out` unused
@@ -97,10 +97,10 @@ const StreamVariant* find_stream_variant(int R, int W, int KL, int KU, int SV, i
                                         int PREC, int ALT = 0, int ELEM = 0);
 // Tensor maps of a launch's input and output rows; false when the buffers'
 // alignment, strides or M do not allow the streaming layout.
-bool encode_stream_maps(const StreamVariant* v, const JwIO& io, CUtensorMap* in, CUtensorMap* out);
-// es: bytes per stored value (8: FP64, 4: FP32).
+bool encode_stream_maps(const StreamVariant* v, const StreamIO& io, CUtensorMap* in, CUtensorMap* out);
+// es: bytes per stored value (8: FP64, 4: FP32); sets: StreamIO::sets.
 bool encode_row_maps(int R, int LIN, int LOUT, int IB, int IBO, const JwIO& io, CUtensorMap* in, CUtensorMap* out,
-                     int es = 8);
+                     int es = 8, int64_t sets = 0);
 
 // Long-system variants: one cluster of C CTAs per system, each CTA a slice of
 // 32*W*R rows (real systems, FP64).
@@ -168,7 +168,7 @@ struct SeqStepsVariant {
     int max_threads;
     const void* func;
     void (*launch)(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const CUtensorMap* in, const CUtensorMap* out,
-                   const JwSteps& S, const JwIO& io);
+                   const JwSteps& S, const JwIO& io, int NW);  // NW: sweeping warps
 };
 const SeqStepsVariant* find_seq_steps_variant(int UB, int MV, int SV, int K, int CH);
 size_t seq_steps_smem_bytes(int K, int64_t Mtab, int NW, int CH);

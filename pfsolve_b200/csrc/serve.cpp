@@ -304,7 +304,7 @@ void launch_flight(PfSolveServer* s, Flight& fl, int cls)
             for (Req* r : fl.reqs) {
                 const ServeOp& o = s->ops[r->r.op];
                 fl.h_entries[e].op = make_operator(s, o, r->r);
-                fl.h_entries[e].io = make_io(o, r->r);
+                fl.h_entries[e].io = StreamIO(make_io(o, r->r));
                 for (int64_t y0 = 0; y0 < r->r.nrhs; y0 += spi) {
                     fl.h_items[k].entry = e;
                     fl.h_items[k].pad = 0;

@@ -47,9 +47,9 @@ const StepsVariant* find_steps_variant(int R, int KL, int KU, int SV, int MV)
 
 template <int UB, bool MV, bool SV, int K, int CH>
 static void seq_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const CUtensorMap* in,
-                          const CUtensorMap* out, const JwSteps& S, const JwIO& io)
+                          const CUtensorMap* out, const JwSteps& S, const JwIO& io, int NW)
 {
-    jw_steps_seq_kernel<UB, MV, SV, K, CH><<<grid, block, smem, st>>>(*in, *out, S, io);
+    jw_steps_seq_kernel<UB, MV, SV, K, CH><<<grid, block, smem, st>>>(*in, *out, S, io, NW);
 }
 
 #define PFB_SQC(UB, MV, SV, K, CH)                                                                            \

@@ -24,7 +24,7 @@ inline int st_threads_fn(int G)
 
 template <class C>
 inline void st_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const CUtensorMap* in,
-                         const CUtensorMap* out, const JwOperator& op, const JwIO& io)
+                         const CUtensorMap* out, const JwOperator& op, const StreamIO& io)
 {
     jw_stream_kernel<C><<<grid, block, smem, st>>>(*in, *out, op, io);
 }
@@ -32,7 +32,7 @@ inline void st_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st, co
 // Element copies in place of tensor copies (jw_stream_elem_kernel).
 template <class C>
 inline void st_elem_launch_fn(dim3 grid, dim3 block, size_t smem, cudaStream_t st, const CUtensorMap*,
-                              const CUtensorMap*, const JwOperator& op, const JwIO& io)
+                              const CUtensorMap*, const JwOperator& op, const StreamIO& io)
 {
     jw_stream_elem_kernel<C><<<grid, block, smem, st>>>(op, io);
 }

@@ -109,13 +109,13 @@ bool encode_rows(CUtensorMap* map, const void* base, int64_t inner, int64_t chun
 }  // namespace
 
 bool encode_row_maps(int R_, int LIN, int LOUT, int IB, int IBO, const JwIO& io, CUtensorMap* in, CUtensorMap* out,
-                     int es)
+                     int es, int64_t pair_sets)
 {
     const int64_t R = R_, M = io.M;
     if (M % R != 0 || io.nsys < 1) return false;
     const int64_t chunks = M / R;
     const bool cplx = LIN != LAY_REAL;
-    const int64_t sets = cplx ? (io.sets ? io.sets : 2 * io.nsys) : io.nsys;
+    const int64_t sets = cplx ? (pair_sets ? pair_sets : 2 * io.nsys) : io.nsys;
     const char* in0 = reinterpret_cast<const char*>(io.in) + io.in_off * es;
     char* out0 = reinterpret_cast<char*>(io.out);
     if (!encode_rows(in, in0, R, chunks, sets, io.in_stride * es, IB, es)) return false;
@@ -180,9 +180,9 @@ bool encode_batch_seq_maps(const JwIO& io, BatchSeqEntry* e)
     return true;
 }
 
-bool encode_stream_maps(const StreamVariant* v, const JwIO& io, CUtensorMap* in, CUtensorMap* out)
+bool encode_stream_maps(const StreamVariant* v, const StreamIO& io, CUtensorMap* in, CUtensorMap* out)
 {
-    return encode_row_maps(v->R, v->LIN, v->LOUT, v->IB, v->IBO, io, in, out, prec_f32_storage(v->PREC) ? 4 : 8);
+    return encode_row_maps(v->R, v->LIN, v->LOUT, v->IB, v->IBO, io, in, out, prec_f32_storage(v->PREC) ? 4 : 8, io.sets);
 }
 
 unsigned stream_status_fetch_clear()
