@@ -435,6 +435,13 @@ PFSOLVE_API PfSolveResult PfSolveBatchGetShape(const PfSolveBatch* batch, int* r
  * warps per CTA (all 0 when the batch runs the group kernel). */
 PFSOLVE_API PfSolveResult PfSolveBatchGetSweepShape(const PfSolveBatch* batch, int* rowsPerChunk, int* buffers,
                                                     int* warpsPerCTA);
+/* The kernel the batch's launches run on. */
+enum {
+    PFSOLVE_BATCH_GROUP = 0,    /* jw_batch_kernel: a group of warps per system */
+    PFSOLVE_BATCH_SWEEP = 1,    /* jw_batch_seq_kernel: one complex system per lane */
+    PFSOLVE_BATCH_STREAMING = 2 /* jw_batch_stream_kernel: a CTA per item, its table built once */
+};
+PFSOLVE_API PfSolveResult PfSolveBatchGetKernel(const PfSolveBatch* batch, int* kernel);
 PFSOLVE_API void PfSolveBatchDestroy(PfSolveBatch* batch);
 
 /* One uneven batch, as PfSolveBatchCreate + PfSolveBatchAppend +
@@ -462,8 +469,9 @@ PFSOLVE_API void PfSolveBatchDestroy(PfSolveBatch* batch);
  * being captured returns PFSOLVE_ERROR_INVALID_ARGUMENT and enqueues nothing;
  * do not issue it under stream capture.
  * The caller's current device is the same on return as on entry.  Results
- * equal PfSolveBatchAppend's for the same descriptor, rows per thread and
- * systems per item. */
+ * equal PfSolveBatchAppend's for the same descriptor with rows per thread and
+ * systems per item set (left 0, a batch plan may choose another kernel, whose
+ * results agree within rounding). */
 #define PFSOLVE_NOALLOC_MAX_ENTRIES 1024
 #define PFSOLVE_NOALLOC_MAX_ITEMS 16384
 PFSOLVE_API PfSolveResult PfSolveBatchAppendNoAlloc(CUdevice device, const PfSolveBatchDesc* desc,
@@ -506,7 +514,9 @@ PFSOLVE_API PfSolveResult PfSolveGetDeviceStatus(void);
  * No counterpart in the reference. */
 PFSOLVE_API PfSolveResult PfSolveGetShape(const PfSolveApplication* app, int* streaming, int* rowsPerThread,
                                           int* warpsPerSystem, int* groupsPerCTA);
-/* Launches that ran on the streaming kernel since load (all apps). */
+/* Launches that ran on the streaming kernel by tensor copies, and on the long-
+ * system and sweep kernels, since load (all apps).  Launches by element copies
+ * are not counted (PfSolveGetLastLaunchForm tells them apart). */
 PFSOLVE_API uint64_t PfSolveStreamingLaunchCount(void);
 
 /* The kernel instance of the most recent launch this library enqueued from
@@ -543,6 +553,11 @@ typedef struct {
     int64_t gridCTAs;   /* CTAs of the (last) kernel of the launch */
 } PfSolveLaunchInfo;
 PFSOLVE_API PfSolveResult PfSolveGetLastLaunch(PfSolveLaunchInfo* info);
+/* The form of that launch where it ran on the streaming kernel: systemsPerGroup
+ * 2 when it solved real systems two at a time, else 1; elementCopies 1 when its
+ * rows moved by element copies, 0 by tensor copies.  Other kernels: 1 and 0.
+ * No counterpart in the reference. */
+PFSOLVE_API PfSolveResult PfSolveGetLastLaunchForm(int* systemsPerGroup, int* elementCopies);
 
 /* ---- Serving engine.  No counterpart in the reference (whose callers drive
  * one application at a time): JW-step requests of mixed size and precision are

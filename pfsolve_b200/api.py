@@ -122,7 +122,8 @@ class App:
 
 
 def streaming_launch_count() -> int:
-    """Launches that ran on the streaming kernel (``PfSolveStreamingLaunchCount``)."""
+    """Launches by tensor copies on the streaming kernel, and on the long-system
+    and sweep kernels (``PfSolveStreamingLaunchCount``)."""
     return int(capi.load().PfSolveStreamingLaunchCount())
 
 
@@ -131,6 +132,13 @@ def last_launch() -> dict:
     info = capi.PfSolveLaunchInfo()
     check(capi.load().PfSolveGetLastLaunch(ctypes.byref(info)), "PfSolveGetLastLaunch")
     return {k: getattr(info, k) for k, _ in info._fields_}
+
+
+def last_launch_form() -> dict:
+    """The form of that launch on the streaming kernel (``PfSolveGetLastLaunchForm``)."""
+    n, elem = ctypes.c_int(), ctypes.c_int()
+    check(capi.load().PfSolveGetLastLaunchForm(ctypes.byref(n), ctypes.byref(elem)), "PfSolveGetLastLaunchForm")
+    return dict(systemsPerGroup=n.value, elementCopies=elem.value)
 
 
 def device_status() -> int:
@@ -205,6 +213,12 @@ class Batch:
               "PfSolveBatchGetSweepShape")
         return dict(rowsPerThread=r.value, warpsPerSystem=w.value, systemsPerItem=spi.value, items=items.value,
                     tunedMs=ms.value, sweepRows=ch.value, sweepBuffers=nb.value, sweepWarps=nw.value)
+
+    def kernel(self) -> int:
+        """PFSOLVE_BATCH_GROUP, _SWEEP or _STREAMING (``PfSolveBatchGetKernel``)."""
+        k = ctypes.c_int()
+        check(self._lib.PfSolveBatchGetKernel(self.handle, ctypes.byref(k)), "PfSolveBatchGetKernel")
+        return k.value
 
     def close(self):
         if getattr(self, "handle", None):

@@ -137,6 +137,7 @@ class PfSolveLaunchInfo(ctypes.Structure):
 PFSOLVE_KERNEL_NONE, PFSOLVE_KERNEL_GROUP, PFSOLVE_KERNEL_STREAMING, PFSOLVE_KERNEL_LONG = 0, 1, 2, 3
 PFSOLVE_KERNEL_CLUSTER, PFSOLVE_KERNEL_STEPS, PFSOLVE_KERNEL_STEPS_SWEEP = 4, 5, 6
 PFSOLVE_KERNEL_DGBMV, PFSOLVE_KERNEL_BLOCK, PFSOLVE_KERNEL_DCT = 7, 8, 9
+PFSOLVE_BATCH_GROUP, PFSOLVE_BATCH_SWEEP, PFSOLVE_BATCH_STREAMING = 0, 1, 2
 
 
 class PfSolveServerStats(ctypes.Structure):
@@ -172,6 +173,7 @@ SIGNATURES = {
     "PfSolveGetShape": (c_int, [_APP_P] + [ctypes.POINTER(c_int)] * 4),
     "PfSolveStreamingLaunchCount": (u64, []),
     "PfSolveGetLastLaunch": (c_int, [ctypes.POINTER(PfSolveLaunchInfo)]),
+    "PfSolveGetLastLaunchForm": (c_int, [ctypes.POINTER(c_int)] * 2),
     "PfSolveServerCreate": (c_int, [ctypes.POINTER(ctypes.c_void_p), ctypes.POINTER(PfSolveServerDesc)]),
     "PfSolveServerAddOperator": (c_int, [ctypes.c_void_p, i64, ctypes.c_void_p, c_int, c_int,
                                          ctypes.POINTER(c_int)]),
@@ -186,6 +188,7 @@ SIGNATURES = {
     "PfSolveBatchAutotune": (c_int, [ctypes.c_void_p, ctypes.c_void_p, c_int]),
     "PfSolveBatchGetShape": (c_int, [ctypes.c_void_p] + [ctypes.POINTER(c_int)] * 4 + [ctypes.POINTER(ctypes.c_double)]),
     "PfSolveBatchGetSweepShape": (c_int, [ctypes.c_void_p] + [ctypes.POINTER(c_int)] * 3),
+    "PfSolveBatchGetKernel": (c_int, [ctypes.c_void_p, ctypes.POINTER(c_int)]),
     "PfSolveBatchDestroy": (None, [ctypes.c_void_p]),
     "PfSolveBatchAppendNoAlloc": (c_int, [c_int, ctypes.POINTER(PfSolveBatchDesc), ctypes.POINTER(PfSolveBatchEntry),
                                           c_int, ctypes.c_void_p]),

@@ -124,10 +124,14 @@ AppState* st(PfSolveApplication* app) { return static_cast<AppState*>(app->inter
 // The kernel instance of the calling thread's most recent launch
 // (PfSolveGetLastLaunch).
 thread_local PfSolveLaunchInfo g_last_launch;
+// its form (PfSolveGetLastLaunchForm): systems per group, element copies
+thread_local int g_last_form[2] = {1, 0};
 
 void record_launch(int kernel, int R, int W, int G, int KL, int KU, int sv, int lin, int lout, int scale, int prec,
-                   int alt, int64_t grid)
+                   int alt, int64_t grid, int per_group = 1, int elem = 0)
 {
+    g_last_form[0] = per_group;
+    g_last_form[1] = elem;
     PfSolveLaunchInfo& i = g_last_launch;
     i.kernel = kernel;
     i.rowsPerThread = R;
@@ -839,7 +843,7 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
     rs.groups = G;
     v->launch(dim3((unsigned)grid), dim3(v->threads(G)), v->smem_bytes(G, rs.nbuf), stream, &e->in, &e->out, op, rs);
     record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, G, v->KL, v->KU, v->SV, s->stream_v->LIN, s->stream_v->LOUT,
-                  v->SCALE, v->PREC, v->ALT, grid);
+                  v->SCALE, v->PREC, v->ALT, grid, rs.sets ? 2 : 1, 0);
     return true;
 }
 
@@ -877,7 +881,7 @@ bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t
     v->launch(dim3((unsigned)grid), dim3(v->threads(G)), v->smem_bytes(G, eio.nbuf), stream, nullptr, nullptr, op,
               eio);
     record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, G, v->KL, v->KU, v->SV, s->elem_v->LIN, s->elem_v->LOUT,
-                  v->SCALE, v->PREC, v->ALT, grid);
+                  v->SCALE, v->PREC, v->ALT, grid, eio.sets ? 2 : 1, 1);
     return true;
 }
 
@@ -1341,6 +1345,13 @@ PfSolveResult PfSolveGetLastLaunch(PfSolveLaunchInfo* info)
 {
     if (!info) return PFSOLVE_ERROR_INVALID_ARGUMENT;
     *info = g_last_launch;
+    return PFSOLVE_SUCCESS;
+}
+
+PfSolveResult PfSolveGetLastLaunchForm(int* systemsPerGroup, int* elementCopies)
+{
+    if (systemsPerGroup) *systemsPerGroup = g_last_form[0];
+    if (elementCopies) *elementCopies = g_last_form[1];
     return PFSOLVE_SUCCESS;
 }
 
@@ -2330,6 +2341,14 @@ PfSolveResult PfSolveBatchGetShape(const PfSolveBatch* b, int* R, int* W, int* s
     if (spi) *spi = b->spi;
     if (items) *items = (int)b->items.size();
     if (ms) *ms = b->tuned_ms;
+    return PFSOLVE_SUCCESS;
+}
+
+PfSolveResult PfSolveBatchGetKernel(const PfSolveBatch* b, int* kernel)
+{
+    if (!b) return PFSOLVE_ERROR_PLAN_NOT_INITIALIZED;
+    if (!kernel) return PFSOLVE_ERROR_INVALID_ARGUMENT;
+    *kernel = b->bstream ? PFSOLVE_BATCH_STREAMING : (b->seq ? PFSOLVE_BATCH_SWEEP : PFSOLVE_BATCH_GROUP);
     return PFSOLVE_SUCCESS;
 }
 

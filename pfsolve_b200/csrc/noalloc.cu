@@ -202,7 +202,7 @@ extern "C" PfSolveResult PfSolveBatchAppendNoAlloc(CUdevice device, const PfSolv
     if (cudaDeviceGetAttribute(&maxopt, cudaDevAttrMaxSharedMemoryPerBlockOptin, device) != cudaSuccess)
         return PFSOLVE_ERROR_FAILED_TO_GET_ATTRIBUTE;
 
-    // launch shape: as PfSolveBatchCreate (rows per thread 8, else 4)
+    // launch shape: as PfSolveBatchCreate's group kernel (rows per thread 8, else 4)
     const BatchVariant* v = nullptr;
     int W = 1, G = 1, blocks = 0;
     const int Rs[2] = {desc->rowsPerThread ? desc->rowsPerThread : 8, 4};
