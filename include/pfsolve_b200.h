@@ -371,7 +371,7 @@ PFSOLVE_API PfSolveResult PfSolveAppendChain(PfSolveApplication** apps, PfSolveL
  * Three kernels: the group kernel (a group of warps per system, rowsPerThread
  * rows per thread), the streaming solve for real systems (a CTA per item, its
  * table built once; the default for real systems of at most 2048 rows without
- * accumulation) and the sweep kernel (one complex system per lane, its
+ * accumulation, 1024 for the mixed mode's 3-band matvec with an upper solve) and the sweep kernel (one complex system per lane, its
  * rows in sequence, a warp per item of 32 systems).  sweepRows = 8 or 16
  * asks for the sweep kernel with that many rows per staged chunk
  * (PFSOLVE_ERROR_UNSUPPORTED_COMBINATION where the batch does not allow it).

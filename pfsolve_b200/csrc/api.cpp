@@ -1970,9 +1970,11 @@ PfSolveResult batch_configure_stream(PfSolveBatch* b)
         b->Mmax > batch_stream_max_rows())
         return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
     const BatchStreamVariant* v = find_batch_stream_variant(b->KL, b->KU, b->SV, b->PREC);
-    if (!v || v->smem_bytes > 227 * 1024 || !allow_max_smem(v->func)) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
+    // (the mixed mode's 3-band kind beyond 1 024 rows: its table leaves the staging buffers no room)
+    if (!v || v->smem_bytes(b->Mmax) > 227 * 1024 || !allow_max_smem(v->func))
+        return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
     int blocks = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, v->func, 512, v->smem_bytes) != cudaSuccess ||
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, v->func, 512, v->smem_bytes(b->Mmax)) != cudaSuccess ||
         blocks < 1) {
         cudaGetLastError();
         return PFSOLVE_ERROR_FAILED_TO_GET_ATTRIBUTE;
@@ -2046,7 +2048,8 @@ PfSolveResult batch_launch(PfSolveBatch* b, cudaStream_t stream)
         const int grid = std::min(nitems, b->max_blocks);
         if (nitems > grid && cudaMemsetAsync(b->d_counter, 0, sizeof(unsigned int), stream) != cudaSuccess)
             return PFSOLVE_ERROR_FAILED_TO_LAUNCH_KERNEL;
-        b->bstream->launch(dim3((unsigned)grid), stream, b->d_entries, b->d_items, nitems, b->d_counter);
+        b->bstream->launch(dim3((unsigned)grid), stream, b->d_entries, b->d_items, nitems, b->d_counter,
+                           b->Mmax);
         g_launches.fetch_add(1, std::memory_order_relaxed);
         if (cudaPeekAtLastError() != cudaSuccess) {
             cudaGetLastError();

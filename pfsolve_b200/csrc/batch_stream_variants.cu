@@ -8,14 +8,22 @@ namespace pfb {
 
 template <class CF>
 static void bs_launch_fn(dim3 grid, cudaStream_t st, const BatchEntryDev* entries, const WorkItem* items, int nitems,
-                         unsigned int* counter)
+                         unsigned int* counter, int64_t Mmax)
 {
-    jw_batch_stream_kernel<CF><<<grid, kBsThreads, bs_smem_bytes<CF>(), st>>>(entries, items, nitems, counter);
+    jw_batch_stream_kernel<CF><<<grid, kBsThreads, bs_smem_bytes<CF>(Mmax), st>>>(entries, items, nitems, counter,
+                                                                                 (int)bs_table_bytes<CF>(Mmax));
+}
+
+template <class CF>
+static size_t bs_smem_fn(int64_t Mmax)
+{
+    static_assert(bs_smem_bytes<CF>(1024) <= 227 * 1024, "every compiled kind runs batches of up to 1 024 rows");
+    return bs_smem_bytes<CF>(Mmax);
 }
 
 #define PFB_BST(KL, KU, SV, P)                                                                                    \
     BatchStreamVariant{KL, KU, SV, P, (const void*)&jw_batch_stream_kernel<BsCfg<KL, KU, SV, P>>,                \
-                       bs_smem_bytes<BsCfg<KL, KU, SV, P>>(), &bs_launch_fn<BsCfg<KL, KU, SV, P>>}
+                       &bs_smem_fn<BsCfg<KL, KU, SV, P>>, &bs_launch_fn<BsCfg<KL, KU, SV, P>>}
 
 static const BatchStreamVariant kBatchStreamVariants[] = {
     PFB_BST(1, 1, SV_UPPER, PREC_F64),

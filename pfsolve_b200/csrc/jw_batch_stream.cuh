@@ -29,7 +29,7 @@ struct BsCfg {
 
 // Shape index of M rows (kBsShapes: longer systems do not run here).
 constexpr int kBsShapes = 5;
-__host__ __device__ inline int bs_shape(int64_t M)
+__host__ __device__ constexpr int bs_shape(int64_t M)
 {
     return M <= 128 ? 0 : (M <= 256 ? 1 : (M <= 512 ? 2 : (M <= 1024 ? 3 : (M <= 2048 ? 4 : kBsShapes))));
 }
@@ -41,20 +41,27 @@ constexpr int kBsBars = kBsBufs * (kBsWarps + kBsWarps / 2 + kBsWarps / 4);
 
 // Shared memory: descriptor | item slots | barriers | scratch | table |
 // (align 1024) | staging buffers (every shape's groups fill the same bytes per
-// warp at 16 rows per thread).
+// warp at 16 rows per thread).  The table holds the shapes up to the longest
+// entry's (Mmax rows): beside the staging buffers the four-warp table of six
+// planes does not fit, so the mixed mode's 3-band kind runs here up to 1 024
+// rows.  It is at least the exchange area the table build borrows from it.
 template <class CF>
-__host__ __device__ constexpr size_t bs_table_bytes()
+__host__ __device__ constexpr size_t bs_table_bytes(int64_t Mmax)
 {
-    size_t t = CF::template St<16, 4>::TBL;
-    if (CF::template St<16, 2>::TBL > t) t = CF::template St<16, 2>::TBL;
+    size_t t = (size_t)kBsWarps * kScratchPerWarp * sizeof(double);
+    const size_t by_shape[kBsShapes] = {CF::template St<4, 1>::TBL, CF::template St<8, 1>::TBL,
+                                        CF::template St<16, 1>::TBL, CF::template St<16, 2>::TBL,
+                                        CF::template St<16, 4>::TBL};
+    for (int k = 0; k < kBsShapes && k <= bs_shape(Mmax); ++k)
+        if (by_shape[k] > t) t = by_shape[k];
     return (t + 15) / 16 * 16;
 }
 constexpr size_t kBsHead = (sizeof(BatchEntryDev) + 15) / 16 * 16 + 16 + (size_t)kBsBars * 8 +
                            (size_t)kBsWarps * kScratchPerWarp * sizeof(double);
 template <class CF>
-__host__ __device__ constexpr size_t bs_smem_bytes()
+__host__ __device__ constexpr size_t bs_smem_bytes(int64_t Mmax)
 {
-    return kBsHead + bs_table_bytes<CF>() + 1024 + (size_t)kBsWarps * kBsBufs * 32 * 16 * sizeof(double);
+    return kBsHead + bs_table_bytes<CF>(Mmax) + 1024 + (size_t)kBsWarps * kBsBufs * 32 * 16 * sizeof(double);
 }
 
 // One item on groups of shape C; bi and par are this group's buffer and phase
@@ -94,7 +101,8 @@ template <class CF>
 __global__ void __launch_bounds__(kBsThreads, 1) jw_batch_stream_kernel(const BatchEntryDev* __restrict__ entries,
                                                                        const WorkItem* __restrict__ items,
                                                                        const int nitems,
-                                                                       unsigned int* __restrict__ counter)
+                                                                       unsigned int* __restrict__ counter,
+                                                                       const int table_bytes)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     BatchEntryDev& e = *reinterpret_cast<BatchEntryDev*>(smem_raw);
@@ -102,7 +110,7 @@ __global__ void __launch_bounds__(kBsThreads, 1) jw_batch_stream_kernel(const Ba
     uint64_t* bars = reinterpret_cast<uint64_t*>(slot + 4);
     double* scratch_all = reinterpret_cast<double*>(bars + kBsBars);
     unsigned char* table = smem_raw + kBsHead;
-    unsigned char* after = table + bs_table_bytes<CF>();
+    unsigned char* after = table + table_bytes;
     unsigned char* bufs = after + ((1024u - (smem_u32(after) & 1023u)) & 1023u);
     uint64_t* bars2 = bars + kBsBufs * kBsWarps;
     uint64_t* bars4 = bars2 + kBsBufs * (kBsWarps / 2);

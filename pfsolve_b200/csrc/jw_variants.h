@@ -38,9 +38,9 @@ const BatchVariant* find_batch_variant(int R, int KL, int KU, int SV, int LIN, i
 struct BatchStreamVariant {
     int KL, KU, SV, PREC;
     const void* func;
-    size_t smem_bytes;
+    size_t (*smem_bytes)(int64_t Mmax);  // Mmax: rows of the longest entry
     void (*launch)(dim3 grid, cudaStream_t st, const BatchEntryDev* entries, const WorkItem* items, int nitems,
-                   unsigned int* counter);
+                   unsigned int* counter, int64_t Mmax);
 };
 const BatchStreamVariant* find_batch_stream_variant(int KL, int KU, int SV, int PREC);
 int batch_stream_shape(int64_t M);            // 0 .. 4: padded rows 128, 256, 512, 1 024, 2 048

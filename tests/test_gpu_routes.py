@@ -49,7 +49,7 @@ def test_pairs_where_compiled(M, R, W, prec):
         assert info["kernel"] == capi.PFSOLVE_KERNEL_GROUP and form == dict(systemsPerGroup=1, elementCopies=0)
 
 
-BATCH_KINDS = [(2, 13, 0, 0), (0, 13, 0, 0), (0, 13, 3, 0), (2, 13, 0, 2), (0, 13, 0, 2), (1, 13, 0, 2), (1, 10, 0, 2),
+BATCH_KINDS = [(2, 13, 0, 0), (0, 13, 0, 0), (0, 13, 3, 0), (0, 13, 3, 2), (2, 13, 0, 2), (0, 13, 0, 2), (1, 13, 0, 2), (1, 10, 0, 2),
                (0, 10, 0, 2)]
 
 
@@ -69,7 +69,9 @@ def test_batch_kernel(ub, jwt, lda, refine):
         kw = dict(upperBanded=ub, jw_type=jwt, mixedPrecisionRefinement=refine)
         if lda:
             kw.update(LDA=lda, KU=1, KL=1)
-        for extra, kernel in ((dict(), capi.PFSOLVE_BATCH_STREAMING), (dict(rowsPerThread=8), capi.PFSOLVE_BATCH_GROUP)):
+        # (the mixed mode's 3-band kind beyond 1 024 rows: the group kernel)
+        chosen = capi.PFSOLVE_BATCH_GROUP if lda and refine and max(Ms) > 1024 else capi.PFSOLVE_BATCH_STREAMING
+        for extra, kernel in ((dict(), chosen), (dict(rowsPerThread=8), capi.PFSOLVE_BATCH_GROUP)):
             b = Batch(ents, **kw, **extra)
             assert b.kernel() == kernel, (Ms, extra)
             b.append()
