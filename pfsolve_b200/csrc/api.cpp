@@ -1935,6 +1935,12 @@ PfSolveResult batch_configure_seq(PfSolveBatch* b, int shape)
     return PFSOLVE_SUCCESS;
 }
 
+// The group kernel's items: about 4 per resident group keep the queue balanced.
+int64_t default_systems_per_item(int64_t systems, int64_t groups)
+{
+    return std::max<int64_t>(8, std::min<int64_t>(256, systems / (4 * groups) + 1));
+}
+
 PfSolveResult batch_configure(PfSolveBatch* b, int R)
 {
     int64_t W = (b->Mmax + 32 * (int64_t)R - 1) / (32 * (int64_t)R);
@@ -1961,10 +1967,123 @@ PfSolveResult batch_configure(PfSolveBatch* b, int R)
 
 // Real systems of at most 2 048 rows on the streaming solve.  An item costs
 // one table build plus its systems, taken a round of a CTA's groups at a time;
-// the entries are cut into items of about equal cost: the cut whose greedy
-// schedule over the SMs (largest item first, as the device's queue hands them
-// out) ends earliest.
-PfSolveResult batch_configure_stream(PfSolveBatch* b)
+// the entries are cut into items of about equal cost.
+
+// Microseconds of an SM per system (batches that fill the chip; the mixed
+// mode's, FP64 takes about 0.55 of them) and per table build, by the shape
+// (padded rows 128, 256, 512, 1 024, 2 048) of an entry's groups.
+constexpr double kStreamSystemUs[5] = {0.13, 0.20, 0.40, 1.25, 2.40}, kStreamBuildUs[5] = {7, 7, 8, 10, 13};
+
+double stream_system_us(const PfSolveBatch* b, int64_t M)
+{
+    return (b->PREC == PREC_MIXED ? 1.0 : 0.55) * kStreamSystemUs[batch_stream_shape(M)];
+}
+
+// Items of equal cost, an entry's whole ones or its last.
+struct ItemRun {
+    double us;
+    int64_t n;
+};
+
+// End of the greedy schedule of the items over `cus` CTAs, largest first, as
+// the device's queue hands them out.
+double schedule_end(std::vector<ItemRun>& runs, int cus)
+{
+    std::sort(runs.begin(), runs.end(), [](const ItemRun& x, const ItemRun& y) { return x.us > y.us; });
+    std::priority_queue<double, std::vector<double>, std::greater<double>> busy;  // CTAs by when they are free
+    double end = 0;
+    for (const ItemRun& r : runs)
+        for (int64_t k = 0; k < r.n; ++k) {
+            double at = 0;
+            if ((int)busy.size() >= cus) {
+                at = busy.top();
+                busy.pop();
+            }
+            busy.push(at + r.us);
+            end = std::max(end, at + r.us);
+        }
+    return end;
+}
+
+// One way to cut the entries: items of `quantum` microseconds of systems.
+// `build`: factor on the table builds.
+void cut_entries(const PfSolveBatch* b, double quantum, double build, std::vector<int>& spi,
+                 std::vector<ItemRun>& runs)
+{
+    runs.clear();
+    for (size_t e = 0; e < b->entries.size(); ++e) {
+        const JwIO& io = b->entries[e].io;
+        const int G = batch_stream_groups(io.M);
+        const double us = stream_system_us(b, io.M), fixed = build * kStreamBuildUs[batch_stream_shape(io.M)];
+        const int64_t rounds = (io.nsys + G - 1) / G;  // of the whole entry
+        const int64_t parts =
+            std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)std::ceil(io.nsys * us / quantum)));
+        const int64_t per = std::max<int64_t>(1, (rounds + parts - 1) / parts);
+        spi[e] = (int)std::min<int64_t>(per * G, INT32_MAX);
+        if (rounds >= per) runs.push_back({fixed + (double)per * G * us, rounds / per});
+        if (rounds % per) runs.push_back({fixed + (double)(rounds % per) * G * us, 1});
+    }
+}
+
+// The cut whose greedy schedule over the SMs ends earliest, out of 46 sizes of
+// item; us: its end with the table builds of the batch's own solve (a
+// bidiagonal table takes about half of a tridiagonal one's time).
+void best_cut(const PfSolveBatch* b, std::vector<int>& best_spi, double& us)
+{
+    std::vector<int> spi(b->entries.size());
+    std::vector<ItemRun> runs;
+    double total = 0, best = 0, best_quantum = 0;
+    for (const BatchEntryDev& e : b->entries) total += (double)e.io.nsys * stream_system_us(b, e.io.M);
+    for (double share = 0.5; share <= 8.0; share *= 1.0625) {
+        const double quantum = std::max(total / b->num_sms / share, 0.5);
+        cut_entries(b, quantum, 1.0, spi, runs);
+        const double end = schedule_end(runs, b->num_sms);
+        if (best_spi.empty() || end < best) {
+            best = end;
+            best_quantum = quantum;
+            best_spi = spi;
+        }
+    }
+    cut_entries(b, best_quantum, b->SV == SV_TRI ? 1.0 : 0.5, spi, runs);
+    us = schedule_end(runs, b->num_sms);
+}
+
+// Microseconds of the same batch on the group kernel's default shape (8 rows
+// per thread, W of a CTA's 8 warps a system): an item costs the coefficients,
+// formed by each group for itself, plus its systems.  Fitted to 428 batches of 1
+// to 1 500 equal entries, 6 % off on average.
+double group_kernel_us(const PfSolveBatch* b)
+{
+    const int W = (int)std::max<int64_t>(1, (b->Mmax + 255) / 256), w = W == 1 ? 0 : (W == 2 ? 1 : 2);
+    const bool tri = b->SV == SV_TRI, mixed = b->PREC == PREC_MIXED;
+    static const double kSystemUs[2][2][3] = {{{1.1, 1.45, 1.45}, {1.9, 2.8, 2.8}},   // bidiagonal: FP64, mixed
+                                              {{1.2, 1.9, 2.1}, {2.3, 4.1, 4.5}}};   // tridiagonal
+    const double us = kSystemUs[tri][mixed][w], build = tri ? 13 : (W <= 2 ? 8 : 11);
+    const BatchVariant* v = find_batch_variant(8, b->KL, b->KU, b->SV, b->LIN, b->LOUT, b->SCALE, b->PREC);
+    const int G = std::max(1, 8 / W);
+    int blocks = 0;
+    if (!v || W > 8 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&blocks, v->func, 32 * W * G,
+                                                                     v->smem_bytes(W, G)) != cudaSuccess) {
+        cudaGetLastError();
+        return HUGE_VAL;
+    }
+    // a second CTA an SM overlaps builds; the systems share the SM
+    const double cta_groups = (double)b->num_sms * G, groups = cta_groups * std::max(blocks, 1);
+    int64_t systems = 0, items = 0, most = 0;
+    for (const BatchEntryDev& e : b->entries) systems += e.io.nsys;
+    const int64_t spi = default_systems_per_item(systems, (int64_t)groups);
+    for (const BatchEntryDev& e : b->entries) {
+        items += (e.io.nsys + spi - 1) / spi;
+        most = std::max(most, std::min(spi, e.io.nsys));
+    }
+    const double item = build + (double)most * us;
+    const double mean = (double)systems * us / cta_groups;
+    if ((double)items <= groups) return std::max(item, build + mean);
+    return (double)items * build / groups + mean + item / 2;
+}
+
+// `always`: without the comparison with the group kernel.
+PfSolveResult batch_configure_stream(PfSolveBatch* b, bool always)
 {
     if (b->LIN != LAY_REAL || b->LOUT != LAY_REAL || b->SCALE || b->entries.empty() ||
         b->Mmax > batch_stream_max_rows())
@@ -1981,52 +2100,19 @@ PfSolveResult batch_configure_stream(PfSolveBatch* b)
     }
     for (const BatchEntryDev& e : b->entries)
         if (e.io.accumulate) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
-    // Microseconds of an SM per system (batches that fill the chip; the mixed
-    // mode's, FP64 takes about 0.55 of them) and per table build, by the shape
-    // (padded rows 128, 256, 512, 1 024, 2 048) of an entry's groups.
-    static const double kSystemUs[5] = {0.13, 0.20, 0.40, 1.25, 2.40}, kBuildUs[5] = {7, 7, 8, 10, 13};
-    const double scale = b->PREC == PREC_MIXED ? 1.0 : 0.55;
-    auto system_us = [&](int64_t M) { return scale * kSystemUs[batch_stream_shape(M)]; };
-    double total = 0;
-    for (const BatchEntryDev& e : b->entries) total += (double)e.io.nsys * system_us(e.io.M);
-    std::vector<int> spi(b->entries.size()), best_spi;
-    std::vector<double> cost;
-    double best = 0;
-    for (double share = 0.5; share <= 8.0; share *= 1.0625) {
-        const double quantum = std::max(total / b->num_sms / share, 0.5);
-        cost.clear();
-        for (size_t e = 0; e < b->entries.size(); ++e) {
-            const JwIO& io = b->entries[e].io;
-            const int G = batch_stream_groups(io.M);
-            const double us = system_us(io.M), build = kBuildUs[batch_stream_shape(io.M)];
-            const int64_t rounds = (io.nsys + G - 1) / G;  // of the whole entry
-            const int64_t parts =
-                std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)std::ceil(io.nsys * us / quantum)));
-            const int64_t per = std::max<int64_t>(1, (rounds + parts - 1) / parts);
-            spi[e] = (int)std::min<int64_t>(per * G, INT32_MAX);
-            for (int64_t r = 0; r < rounds; r += per)
-                cost.push_back(build + (double)std::min(per, rounds - r) * G * us);
-        }
-        std::sort(cost.begin(), cost.end(), std::greater<double>());
-        std::priority_queue<double, std::vector<double>, std::greater<double>> busy;  // CTAs by when they are free
-        double end = 0;
-        for (double c : cost) {
-            double at = 0;
-            if ((int)busy.size() >= b->num_sms) {
-                at = busy.top();
-                busy.pop();
-            }
-            busy.push(at + c);
-            end = std::max(end, at + c);
-        }
-        if (best_spi.empty() || end < best) {
-            best = end;
-            best_spi = spi;
-        }
-    }
+    std::vector<int> spi;
+    double stream_us = 0;
+    best_cut(b, spi, stream_us);
+    // Many entries of few systems: the items of an SM run one after another,
+    // each behind its table build, while the group kernel builds eight an SM at
+    // once.  1 500 entries of one system of 200 rows: 76.8 us here, 25.4 on the
+    // group kernel (bidiagonal 37.6 and 18.9); 400 of 500 rows 29.4 and 17.2;
+    // 64 of 300 systems of 40 rows 23.5 and 58.6.  The estimates' own errors are
+    // the reason for the factor.
+    if (!always && group_kernel_us(b) < 0.85 * stream_us) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
     std::vector<double> us;
-    for (const BatchEntryDev& e : b->entries) us.push_back(system_us(e.io.M));
-    const PfSolveResult r = batch_build_items(b, 1, best_spi.data(), us.data());
+    for (const BatchEntryDev& e : b->entries) us.push_back(stream_system_us(b, e.io.M));
+    const PfSolveResult r = batch_build_items(b, 1, spi.data(), us.data());
     if (r != PFSOLVE_SUCCESS) return r;
     b->bstream = v;
     b->seq = nullptr;
@@ -2036,7 +2122,7 @@ PfSolveResult batch_configure_stream(PfSolveBatch* b)
     if (b->W == 3) b->W = 4;
     b->G = 1;
     b->max_blocks = b->num_sms;
-    b->spi = *std::max_element(best_spi.begin(), best_spi.end());
+    b->spi = *std::max_element(spi.begin(), spi.end());
     return PFSOLVE_SUCCESS;
 }
 
@@ -2204,8 +2290,9 @@ PfSolveResult PfSolveBatchCreate(PfSolveBatch** out, CUdevice device, const PfSo
         *out = b;
         return PFSOLVE_SUCCESS;
     }
-    // real systems of up to 2 048 rows: the streaming solve
-    if (!desc->rowsPerThread && desc->systemsPerItem <= 0 && batch_configure_stream(b) == PFSOLVE_SUCCESS) {
+    // real systems of up to 2 048 rows: the streaming solve, where it is the faster one
+    if (!desc->rowsPerThread && desc->systemsPerItem <= 0 &&
+        batch_configure_stream(b, false) == PFSOLVE_SUCCESS) {
         *out = b;
         return PFSOLVE_SUCCESS;
     }
@@ -2215,11 +2302,9 @@ PfSolveResult PfSolveBatchCreate(PfSolveBatch** out, CUdevice device, const PfSo
     if (r != PFSOLVE_SUCCESS) return fail(r);
     int spi = desc->systemsPerItem;
     if (spi <= 0) {
-        // about 4 items per resident group keeps the queue balanced
         int64_t total = 0;
         for (const auto& e : b->entries) total += e.io.nsys;
-        const int64_t groups = std::max<int64_t>(1, (int64_t)b->max_blocks * b->G);
-        spi = (int)std::max<int64_t>(8, std::min<int64_t>(256, total / (4 * groups) + 1));
+        spi = (int)default_systems_per_item(total, std::max<int64_t>(1, (int64_t)b->max_blocks * b->G));
     }
     if ((r = batch_build_items(b, spi)) != PFSOLVE_SUCCESS) return fail(r);
     *out = b;
@@ -2298,7 +2383,7 @@ PfSolveResult PfSolveBatchAutotune(PfSolveBatch* b, cudaStream_t stream, int ite
             bestShape = shape;
         }
     }
-    if (batch_configure_stream(b) == PFSOLVE_SUCCESS) {
+    if (batch_configure_stream(b, true) == PFSOLVE_SUCCESS) {
         const double per = time_shape();
         if (per < best) {
             best = per;
@@ -2320,7 +2405,7 @@ PfSolveResult PfSolveBatchAutotune(PfSolveBatch* b, cudaStream_t stream, int ite
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
-    PfSolveResult r = bestStream ? batch_configure_stream(b)
+    PfSolveResult r = bestStream ? batch_configure_stream(b, true)
                                  : (bestR ? batch_configure(b, bestR) : batch_configure_seq(b, bestShape));
     if (r == PFSOLVE_SUCCESS && !bestStream) r = batch_build_items(b, bestSpi);
     if (r == PFSOLVE_SUCCESS) b->tuned_ms = best;
