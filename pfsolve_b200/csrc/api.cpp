@@ -1985,67 +1985,132 @@ struct ItemRun {
     int64_t n;
 };
 
-// End of the greedy schedule of the items over `cus` CTAs, largest first, as
-// the device's queue hands them out.
-double schedule_end(std::vector<ItemRun>& runs, int cus)
+// End of the greedy schedule of the items (largest first, as the device's queue
+// hands them out) over `cus` CTAs; runs: sorted.
+double schedule_end(const std::vector<ItemRun>& runs, int cus, std::vector<double>& busy)
 {
-    std::sort(runs.begin(), runs.end(), [](const ItemRun& x, const ItemRun& y) { return x.us > y.us; });
-    std::priority_queue<double, std::vector<double>, std::greater<double>> busy;  // CTAs by when they are free
+    busy.assign(cus, 0.0);  // a heap: when each CTA is free, the first one at [0]
     double end = 0;
     for (const ItemRun& r : runs)
         for (int64_t k = 0; k < r.n; ++k) {
-            double at = 0;
-            if ((int)busy.size() >= cus) {
-                at = busy.top();
-                busy.pop();
+            const double at = busy[0] + r.us;
+            end = std::max(end, at);
+            int p = 0, c = 1;  // its new time sinks into the heap
+            while (c < cus) {
+                if (c + 1 < cus && busy[c + 1] < busy[c]) ++c;
+                if (busy[c] >= at) break;
+                busy[p] = busy[c];
+                p = c;
+                c = 2 * p + 1;
             }
-            busy.push(at + r.us);
-            end = std::max(end, at + r.us);
+            busy[p] = at;
         }
     return end;
 }
 
-// One way to cut the entries: items of `quantum` microseconds of systems.
-// `build`: factor on the table builds.
-void cut_entries(const PfSolveBatch* b, double quantum, double build, std::vector<int>& spi,
-                 std::vector<ItemRun>& runs)
+// What no schedule of the sorted items can beat: of k cus + 1 items some CTA
+// gets k + 1, none of them smaller than the last of these items.
+double pigeonhole_bound(const std::vector<ItemRun>& runs, int cus)
+{
+    double bound = 0;
+    int64_t before = 0;
+    for (const ItemRun& r : runs) {
+        before += r.n;
+        const int64_t k = (before - 1) / cus;  // the run holds item k cus + 1, or an earlier one did
+        if (k * cus >= before - r.n) bound = std::max(bound, (double)(k + 1) * r.us);
+    }
+    return bound;
+}
+
+// An entry as the cuts see it: rounds of its shape's groups, microseconds of
+// its systems, of a round and of a table build.
+struct CutEntry {
+    uint32_t rounds;
+    double work, round_us, build_us;
+};
+
+// Rounds per item of an entry cut into items of `quantum` microseconds of systems.
+uint32_t rounds_per_item(const CutEntry& c, double quantum)
+{
+    if (c.work <= quantum) return std::max(c.rounds, 1u);
+    const uint32_t parts = (uint32_t)std::min<double>(c.rounds, std::ceil(c.work / quantum));
+    return (c.rounds + parts - 1) / parts;
+}
+
+// The items of one cut, largest first; build: factor on the table builds.
+void cut_items(const std::vector<CutEntry>& entries, double quantum, double build, std::vector<ItemRun>& runs)
 {
     runs.clear();
-    for (size_t e = 0; e < b->entries.size(); ++e) {
-        const JwIO& io = b->entries[e].io;
-        const int G = batch_stream_groups(io.M);
-        const double us = stream_system_us(b, io.M), fixed = build * kStreamBuildUs[batch_stream_shape(io.M)];
-        const int64_t rounds = (io.nsys + G - 1) / G;  // of the whole entry
-        const int64_t parts =
-            std::max<int64_t>(1, std::min<int64_t>(rounds, (int64_t)std::ceil(io.nsys * us / quantum)));
-        const int64_t per = std::max<int64_t>(1, (rounds + parts - 1) / parts);
-        spi[e] = (int)std::min<int64_t>(per * G, INT32_MAX);
-        if (rounds >= per) runs.push_back({fixed + (double)per * G * us, rounds / per});
-        if (rounds % per) runs.push_back({fixed + (double)(rounds % per) * G * us, 1});
+    for (const CutEntry& c : entries) {
+        const uint32_t per = rounds_per_item(c, quantum), whole = c.rounds / per, rest = c.rounds - whole * per;
+        if (whole) runs.push_back({build * c.build_us + (double)per * c.round_us, whole});
+        if (rest) runs.push_back({build * c.build_us + (double)rest * c.round_us, 1});
     }
+    std::sort(runs.begin(), runs.end(), [](const ItemRun& x, const ItemRun& y) { return x.us > y.us; });
 }
 
 // The cut whose greedy schedule over the SMs ends earliest, out of 46 sizes of
-// item; us: its end with the table builds of the batch's own solve (a
-// bidiagonal table takes about half of a tridiagonal one's time).
-void best_cut(const PfSolveBatch* b, std::vector<int>& best_spi, double& us)
+// item (ties: the largest); spi: systems per item of each entry; us: its end
+// with the table builds of the batch's own solve (a bidiagonal table takes about
+// half of a tridiagonal one's time).  Every cut has a bound from its items' sum
+// and its largest item; they are taken in its order, with a second bound before
+// a cut is scheduled, so that few are (32 requests: 46 schedules took 320 us of
+// host time, a plan's creation 450 without them).
+void best_cut(const PfSolveBatch* b, std::vector<int>& spi, double& us)
 {
-    std::vector<int> spi(b->entries.size());
+    struct Cut {
+        double bound, quantum;
+        int k;
+    };
+    std::vector<Cut> cuts;
+    std::vector<CutEntry> entries;
     std::vector<ItemRun> runs;
-    double total = 0, best = 0, best_quantum = 0;
-    for (const BatchEntryDev& e : b->entries) total += (double)e.io.nsys * stream_system_us(b, e.io.M);
+    std::vector<double> busy;
+    entries.reserve(b->entries.size());
+    double total = 0;
+    for (const BatchEntryDev& e : b->entries) {
+        const int G = batch_stream_groups(e.io.M);
+        const double one = stream_system_us(b, e.io.M);
+        entries.push_back({(uint32_t)std::min<int64_t>((e.io.nsys + G - 1) / G, INT32_MAX), (double)e.io.nsys * one,
+                           G * one, kStreamBuildUs[batch_stream_shape(e.io.M)]});
+        total += entries.back().work;
+    }
     for (double share = 0.5; share <= 8.0; share *= 1.0625) {
         const double quantum = std::max(total / b->num_sms / share, 0.5);
-        cut_entries(b, quantum, 1.0, spi, runs);
-        const double end = schedule_end(runs, b->num_sms);
-        if (best_spi.empty() || end < best) {
+        double sum = 0, most = 0;
+        for (const CutEntry& c : entries) {
+            const uint32_t per = rounds_per_item(c, quantum), items = (c.rounds + per - 1) / per;
+            sum += items * c.build_us + c.rounds * c.round_us;
+            if (items) most = std::max(most, c.build_us + (double)per * c.round_us);
+        }
+        cuts.push_back({std::max(sum / b->num_sms * (1 - 1e-12), most), quantum, (int)cuts.size()});
+    }
+    auto before = [](const Cut& x, const Cut& y) { return x.bound != y.bound ? x.bound < y.bound : x.k < y.k; };
+    std::sort(cuts.begin(), cuts.end(), before);
+    double best = HUGE_VAL;
+    const Cut* best_of = nullptr;
+    for (const Cut& c : cuts) {
+        if (c.bound > best) break;
+        if (c.bound == best && c.k > best_of->k) continue;
+        cut_items(entries, c.quantum, 1.0, runs);
+        const double bound = pigeonhole_bound(runs, b->num_sms);
+        if (bound > best || (bound == best && c.k > best_of->k)) continue;
+        const double end = schedule_end(runs, b->num_sms, busy);
+        if (end < best || (end == best && c.k < best_of->k)) {
             best = end;
-            best_quantum = quantum;
-            best_spi = spi;
+            best_of = &c;
         }
     }
-    cut_entries(b, best_quantum, b->SV == SV_TRI ? 1.0 : 0.5, spi, runs);
-    us = schedule_end(runs, b->num_sms);
+    spi.clear();
+    for (size_t e = 0; e < entries.size(); ++e)
+        spi.push_back((int)std::min<int64_t>(
+            (int64_t)rounds_per_item(entries[e], best_of->quantum) * batch_stream_groups(b->entries[e].io.M), INT32_MAX));
+    if (b->SV == SV_TRI) {
+        us = best;
+    } else {
+        cut_items(entries, best_of->quantum, 0.5, runs);
+        us = schedule_end(runs, b->num_sms, busy);
+    }
 }
 
 // Microseconds of the same batch on the group kernel's default shape (8 rows
