@@ -13,6 +13,8 @@
 #include <cstring>
 #include <functional>
 #include <map>
+#include <memory>
+#include <mutex>
 #include <new>
 #include <queue>
 #include <tuple>
@@ -34,6 +36,75 @@ enum AppKind { APP_JW = 1, APP_DGBMV = 2, APP_BLOCK = 3, APP_DCT = 4 };
 constexpr int64_t kMaxRows = 4096;       // one CTA group per system (<= 8 warps x 32 x 16 rows)
 constexpr int64_t kMaxRowsLong = 65536;  // JW apps: up to 64 slices of 1024 rows per system (single pass)
 
+// Forms of a JW or dgbmv plan beside the one it is created with: element copies,
+// systems in pairs, the double-double forms by their number.  Each is chosen at
+// the first launch that asks for it (its kernel loaded, its occupancy queried):
+// at every plan's creation they cost 25 to 50 % of its time, and the first plan
+// of a process up to 23 ms of kernel loading.  Launches from several threads may
+// ask at once.
+struct LaunchForms {
+    struct Stream {
+        const StreamVariant* v = nullptr;  // nullptr: not compiled, or it does not fit
+        int G = 0, max_blocks = 0, nbuf = 2;
+    };
+    struct Group {
+        const JwVariant* v = nullptr;
+        int W = 1, G = 1, max_blocks = 0;
+    };
+    // the plan
+    int64_t M = 0;
+    int KL = 0, KU = 0, sv = 0, LIN = 0, LOUT = 0, SCALE = 0, prec = 0, alt = 0;
+    int R_req = 0, nbuf_req = 0, num_sms = 0;
+    bool streams = false;  // the streaming kernel may run (kernelPath, precision)
+    bool dd = false;       // double-double with the caller's rows per thread open
+    const StreamVariant* stream_v = nullptr;
+
+    const Stream& elem()
+    {
+        once(1, [this] { choose_elem(); });
+        return elem_;
+    }
+    const Stream& elem_pair()
+    {
+        once(2, [this] { choose_pair(elem().v, elem_pair_); });
+        return elem_pair_;
+    }
+    const Stream& stream_pair()
+    {
+        once(4, [this] { choose_pair(stream_v, stream_pair_); });
+        return stream_pair_;
+    }
+    const Group& dd_few()
+    {
+        once(8, [this] { choose_dd(4, 0, dd_few_); });
+        return dd_few_;
+    }
+    const Group& dd_many()
+    {
+        once(16, [this] { choose_dd(M <= 128 ? 4 : (M <= 256 ? 8 : 16), 1, dd_many_); });
+        return dd_many_;
+    }
+
+private:
+    template <class F>
+    void once(unsigned bit, F choose)
+    {
+        if (have.load(std::memory_order_acquire) & bit) return;
+        std::lock_guard<std::recursive_mutex> lk(mu);
+        if (have.load(std::memory_order_relaxed) & bit) return;
+        choose();
+        cudaGetLastError();
+        have.fetch_or(bit, std::memory_order_release);
+    }
+    void choose_elem();
+    void choose_pair(const StreamVariant* v, Stream& out);
+    void choose_dd(int R, int tbl, Group& out);
+    std::recursive_mutex mu;  // a pair's choice asks for its single form's
+    std::atomic<unsigned> have{0};
+    Stream elem_, elem_pair_, stream_pair_;
+    Group dd_few_, dd_many_;
+};
+
 struct AppState {
     AppKind kind;
     int num_sms = 0;
@@ -49,20 +120,9 @@ struct AppState {
     // streaming variant (FP64, TMA-staged systems), used when a launch's
     // buffers allow it; `variant` serves the other launches
     const StreamVariant* stream_v = nullptr;
-    // the streaming kernel with element copies, for launches whose rows no
-    // tensor map describes
-    const StreamVariant* elem_v = nullptr;
-    int elem_G = 0, elem_max_blocks = 0, elem_nbuf = 2;
-    // both forms with real systems solved two at a time (nullptr: not compiled)
-    struct Pair {
-        const StreamVariant* v = nullptr;
-        int G = 0, max_blocks = 0, nbuf = 2;
-    } stream_pair, elem_pair;
-    // double-double: the forms for many and for few systems (choose_dd)
-    struct Form {
-        const JwVariant* v = nullptr;
-        int W = 1, G = 1, max_blocks = 0;
-    } dd_many, dd_few;
+    // forms that only some launches of the plan need, chosen by the first of them
+    std::shared_ptr<LaunchForms> forms_own;
+    LaunchForms* forms = nullptr;
     int stream_G = 0, stream_max_blocks = 0;
     int stream_nbuf = 2;  // staging buffers per group
     int nbuf_req = 0;     // caller's staging buffers per group (0: choose)
@@ -108,10 +168,7 @@ struct AppState {
         int R, W, G, max_blocks;
         const StreamVariant* stream_v;
         int stream_G, stream_max_blocks, stream_nbuf;
-        const StreamVariant* elem_v;
-        int elem_G, elem_max_blocks, elem_nbuf;
-        Pair stream_pair, elem_pair;
-        Form dd_many, dd_few;
+        std::shared_ptr<LaunchForms> forms;
     };
     std::vector<ChainPlan> chain_plans;
     // streams
@@ -190,7 +247,7 @@ int pick_rows_per_thread(int64_t M, int requested)
 // faster for FP32 (its 2-KB systems, solved fastest, need more of them
 // in flight), and where they cost groups (the config-2 chain) much
 // slower.
-bool stream_groups(AppState* s, const StreamVariant* v, int* G_out, int* nbuf_out, int* max_blocks)
+bool stream_groups(const StreamVariant* v, int nbuf_req, int num_sms, int* G_out, int* nbuf_out, int* max_blocks)
 {
     const int T = 32 * v->W;
     auto fits = [&](int G, int nb, int* blocks) {
@@ -199,28 +256,27 @@ bool stream_groups(AppState* s, const StreamVariant* v, int* G_out, int* nbuf_ou
         return cudaOccupancyMaxActiveBlocksPerMultiprocessor(blocks, v->func, v->threads(G), smem) == cudaSuccess &&
                *blocks >= 1;
     };
-    const bool req = s->nbuf_req >= 2 && s->nbuf_req <= kStMaxBuffers;
+    const bool req = nbuf_req >= 2 && nbuf_req <= kStMaxBuffers;
     for (int G = std::min(v->max_threads / T, 15); G >= 1; --G) {
         int blocks = 0;
-        int nb = req ? s->nbuf_req : 2;
-        if (!req && s->prec == PREC_F32 && fits(G, 3, &blocks)) nb = 3;
+        int nb = req ? nbuf_req : 2;
+        if (!req && v->PREC == PREC_F32 && fits(G, 3, &blocks)) nb = 3;
         if (!fits(G, nb, &blocks)) continue;
         *G_out = G;
         *nbuf_out = nb;
-        *max_blocks = blocks * s->num_sms;
+        *max_blocks = blocks * num_sms;
         return true;
     }
     return false;
 }
 
 // The form of a real streaming variant that solves systems two at a time.
-void choose_pair(AppState* s, const StreamVariant* v, AppState::Pair& out)
+void LaunchForms::choose_pair(const StreamVariant* v, Stream& out)
 {
-    out = AppState::Pair();
     if (!v || v->LIN != LAY_REAL || v->ALT || v->SCALE) return;
     const StreamVariant* p =
         find_stream_variant(v->R, v->W, v->KL, v->KU, v->SV, LAY_XXII, LAY_XXII, 0, v->PREC, 0, v->ELEM);
-    if (p && stream_groups(s, p, &out.G, &out.nbuf, &out.max_blocks)) out.v = p;
+    if (p && stream_groups(p, nbuf_req, num_sms, &out.G, &out.nbuf, &out.max_blocks)) out.v = p;
 }
 
 // The streaming kernel with element copies for a plan that has a group-kernel
@@ -228,24 +284,43 @@ void choose_pair(AppState* s, const StreamVariant* v, AppState::Pair& out)
 // offsets, row counts that the rows per thread do not divide) take it instead
 // of the group kernel.  The shortest compiled capacity that holds M rows: 4,
 // 8, then 16 rows per thread of one warp, 16 of two and four warps, 32 of four.
-void choose_elem(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
+void LaunchForms::choose_elem()
 {
-    s->elem_v = nullptr;
-    s->elem_pair = AppState::Pair();
-    if ((s->prec != PREC_F64 && s->prec != PREC_MIXED && !prec_f32_storage(s->prec)) || s->no_stream) return;
-    if (s->alt && s->prec != PREC_F64) return;
+    if (!streams || (alt && prec != PREC_F64)) return;
     static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 2}, {32, 4}};
     for (const auto& rw : shapes) {
-        if (32 * (int64_t)rw[0] * rw[1] < M || (s->R_req && rw[0] != s->R_req)) continue;
-        const StreamVariant* v =
-            find_stream_variant(rw[0], rw[1], s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, s->alt, 1);
-        if (v && stream_groups(s, v, &s->elem_G, &s->elem_nbuf, &s->elem_max_blocks)) {
-            s->elem_v = v;
-            choose_pair(s, v, s->elem_pair);
+        if (32 * (int64_t)rw[0] * rw[1] < M || (R_req && rw[0] != R_req)) continue;
+        const StreamVariant* v = find_stream_variant(rw[0], rw[1], KL, KU, sv, LIN, LOUT, SCALE, prec, alt, 1);
+        if (v && stream_groups(v, nbuf_req, num_sms, &elem_.G, &elem_.nbuf, &elem_.max_blocks)) {
+            elem_.v = v;
             break;
         }
     }
-    cudaGetLastError();
+}
+
+bool stream_precision(int prec) { return prec == PREC_F64 || prec == PREC_MIXED || prec_f32_storage(prec); }
+
+// The plan's further forms, none of them chosen yet.
+void set_forms(AppState* s, int64_t M, int LIN, int LOUT, int SCALE, bool dd = false)
+{
+    s->forms_own = std::make_shared<LaunchForms>();
+    LaunchForms& f = *s->forms_own;
+    f.M = M;
+    f.KL = s->KL;
+    f.KU = s->KU;
+    f.sv = s->sv;
+    f.LIN = LIN;
+    f.LOUT = LOUT;
+    f.SCALE = SCALE;
+    f.prec = s->prec;
+    f.alt = s->alt;
+    f.R_req = s->R_req;
+    f.nbuf_req = s->nbuf_req;
+    f.num_sms = s->num_sms;
+    f.streams = stream_precision(s->prec) && !s->no_stream;
+    f.dd = dd;
+    f.stream_v = s->stream_v;
+    s->forms = &f;
 }
 
 // Streaming variant for M rows: rows per thread R (the caller's choice, else
@@ -255,8 +330,7 @@ void choose_elem(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
 bool choose_stream(AppState* s, int64_t M, int LIN, int LOUT, int SCALE, bool alt = false)
 {
     s->stream_v = nullptr;
-    s->stream_pair = AppState::Pair();
-    if ((s->prec != PREC_F64 && s->prec != PREC_MIXED && !prec_f32_storage(s->prec)) || s->no_stream) return false;
+    if (!stream_precision(s->prec) || s->no_stream) return false;
     int cand[3][2];
     int n = 0;
     const int prefs[3] = {16, 32, 8};
@@ -279,9 +353,8 @@ bool choose_stream(AppState* s, int64_t M, int LIN, int LOUT, int SCALE, bool al
         const StreamVariant* v =
             find_stream_variant(cand[i][0], cand[i][1], s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, alt);
         if (!v) continue;
-        if (stream_groups(s, v, &s->stream_G, &s->stream_nbuf, &s->stream_max_blocks)) {
+        if (stream_groups(v, s->nbuf_req, s->num_sms, &s->stream_G, &s->stream_nbuf, &s->stream_max_blocks)) {
             s->stream_v = v;
-            choose_pair(s, v, s->stream_pair);
             return true;
         }
     }
@@ -545,13 +618,10 @@ PfSolveResult plan_alt(AppState* s, const PfSolveConfiguration& c, int base_prec
     // (partial output windows, unaligned rows) and kernelPath 1.
     s->no_stream = c.kernelPath == 1;
     if (s->prec == PREC_F64) choose_stream(s, M, LAY_REAL, LAY_REAL, 0, true);
-    choose_elem(s, M, LAY_REAL, LAY_REAL, 0);
+    set_forms(s, M, LAY_REAL, LAY_REAL, 0);
     return PFSOLVE_SUCCESS;
 }
 
-// Pick the kernel variant and launch shape for M rows: register variants
-// first, then coefficient-table variants (FP64); rows per thread from the
-// caller's choice (s->R) first, then the other compiled choices.
 // Double-double launches of a table-form plan whose rows per thread the caller
 // left open.  Many systems: the table form with the shortest capacity that
 // holds M rows -- 4, 8 and 16 rows per thread of one warp, 16 of two (2^23
@@ -560,21 +630,18 @@ PfSolveResult plan_alt(AppState* s, const PfSolveConfiguration& c, int base_prec
 // 1 000 174 and 140).  Up to three rounds of its resident groups: the register
 // form at 4 rows per thread, whose prologue and solve are the shortest (8
 // systems: N = 512 13.5 against 22.8 us, 1 000 17.7 against 24).
-void choose_dd(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
+void LaunchForms::choose_dd(int R, int tbl, Group& f)
 {
-    auto take = [&](int R, int tbl, AppState::Form& f) {
-        const int64_t W = (M + 32 * (int64_t)R - 1) / (32 * (int64_t)R);
-        const JwVariant* v = find_jw_variant(R, s->KL, s->KU, s->sv, LIN, LOUT, SCALE, s->prec, tbl);
-        if (!v || W > 8 || 32 * W > v->max_threads || !choose_groups(v, (int)W, s->num_sms, f.G, f.max_blocks)) return;
-        f.v = v;
-        f.W = (int)W;
-    };
-    if (M > 1024) return;
-    take(M <= 128 ? 4 : (M <= 256 ? 8 : 16), 1, s->dd_many);
-    take(4, 0, s->dd_few);
-    cudaGetLastError();
+    const int64_t W = (M + 32 * (int64_t)R - 1) / (32 * (int64_t)R);
+    const JwVariant* v = find_jw_variant(R, KL, KU, sv, LIN, LOUT, SCALE, prec, tbl);
+    if (!v || W > 8 || 32 * W > v->max_threads || !choose_groups(v, (int)W, num_sms, f.G, f.max_blocks)) return;
+    f.v = v;
+    f.W = (int)W;
 }
 
+// Pick the kernel variant and launch shape for M rows: register variants
+// first, then coefficient-table variants (FP64); rows per thread from the
+// caller's choice (s->R) first, then the other compiled choices.
 PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCALE)
 {
     // Double-double: the table form first (16 rows per thread where a system
@@ -598,7 +665,7 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
             s->W = (int)W;
             s->G = G;
             s->max_blocks = maxb;
-            if (!s->R_req) choose_dd(s, M, LIN, LOUT, SCALE);
+            set_forms(s, M, LIN, LOUT, SCALE, !s->R_req && M <= 1024);
             return PFSOLVE_SUCCESS;
         }
     }
@@ -618,7 +685,7 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
             if (!choose_groups(v, (int)W, s->num_sms, G, maxb)) continue;
             s->variant = v;
             choose_stream(s, M, LIN, LOUT, SCALE);
-            choose_elem(s, M, LIN, LOUT, SCALE);
+            set_forms(s, M, LIN, LOUT, SCALE);
             s->R = R;
             s->W = (int)W;
             s->G = G;
@@ -630,7 +697,10 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
     // systems, a cluster plan), whose launches need buffers those kernels can
     // take.
     s->variant = nullptr;
-    if (choose_stream(s, M, LIN, LOUT, SCALE)) return PFSOLVE_SUCCESS;
+    if (choose_stream(s, M, LIN, LOUT, SCALE)) {
+        set_forms(s, M, LIN, LOUT, SCALE);
+        return PFSOLVE_SUCCESS;
+    }
     if (M > kMaxRows && choose_long(s, M, LIN, LOUT, SCALE)) return PFSOLVE_SUCCESS;
     if (M > kMaxRows && choose_cluster(s, M, LIN, LOUT, SCALE)) return PFSOLVE_SUCCESS;
     // nothing compiled fits: distinguish "too long" from "not compiled"
@@ -811,7 +881,7 @@ PfSolveResult launch_long(AppState* s, const JwOperator& op, const JwIO& io, cud
 // that every table value read from shared memory (the streaming kernel's bound
 // on real systems) serves two.  Worth it once every resident pair has two
 // rounds of work.
-bool take_pairs(const AppState::Pair& p, StreamIO& io)
+bool take_pairs(const LaunchForms::Stream& p, StreamIO& io)
 {
     if (!p.v || io.nsys < 4 * (int64_t)p.max_blocks * p.G) return false;
     io.sets = io.nsys;
@@ -831,10 +901,14 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
     if (v->ALT) rs.nsys = io.nsys / 2;
     int G = s->stream_G, max_blocks = s->stream_max_blocks;
     rs.nbuf = s->stream_nbuf;
-    if (take_pairs(s->stream_pair, rs)) {
-        v = s->stream_pair.v;
-        G = s->stream_pair.G;
-        max_blocks = s->stream_pair.max_blocks;
+    // (fewer than four systems an SM: no pair form's rule can hold)
+    if (rs.nsys >= 4 * (int64_t)s->num_sms && s->forms) {
+        const LaunchForms::Stream& p = s->forms->stream_pair();
+        if (take_pairs(p, rs)) {
+            v = p.v;
+            G = p.G;
+            max_blocks = p.max_blocks;
+        }
     }
     const MapCacheEntry* e = stream_maps(v, rs);
     if (!e) return false;
@@ -852,13 +926,15 @@ bool launch_stream(AppState* s, const JwOperator& op, const JwIO& io, cudaStream
 // pair's).
 bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t stream)
 {
-    const StreamVariant* v = s->elem_v;
-    if (!v || io.accumulate || io.oz0 > 0 || io.oz1 < io.M) return false;
+    if (!s->forms || !s->forms->streams || io.accumulate || io.oz0 > 0 || io.oz1 < io.M) return false;
     // Few systems: the group kernel's short chunks give the lower latency as
     // long as each of its resident groups solves at most two (N = 1 001 FP64:
     // 592 systems 11.3 against 12.7 us, 1 184 systems 15.2 against 13.0;
     // N = 501: 1 184 systems 10.9 against 11.7, 9 472 systems 37.4 against 25.3).
     if (s->variant && io.nsys <= 2 * (int64_t)s->max_blocks * s->G) return false;
+    const LaunchForms::Stream& single = s->forms->elem();
+    const StreamVariant* v = single.v;
+    if (!v) return false;
     const int es = prec_f32_storage(v->PREC) ? 4 : 8;
     const bool packed = v->LOUT == LAY_PACKED;
     const uintptr_t in0 = reinterpret_cast<uintptr_t>(io.in) + (uintptr_t)io.in_off * es;
@@ -866,21 +942,24 @@ bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t
     if (in0 % es || out0 % (packed ? 2 * es : es)) return false;
     StreamIO eio(io);
     if (v->ALT) eio.nsys = io.nsys / 2;  // row sets, two systems each
-    eio.nbuf = s->elem_nbuf;
+    eio.nbuf = single.nbuf;
     eio.unit16 = in0 % 16 == 0 && (io.in_stride * es) % 16 == 0 &&
                  (packed || (out0 % 16 == 0 && (io.out_stride * es) % 16 == 0));
-    int G = s->elem_G, max_blocks = s->elem_max_blocks;
-    if (take_pairs(s->elem_pair, eio)) {
-        v = s->elem_pair.v;
-        G = s->elem_pair.G;
-        max_blocks = s->elem_pair.max_blocks;
+    int G = single.G, max_blocks = single.max_blocks;
+    if (eio.nsys >= 4 * (int64_t)s->num_sms) {
+        const LaunchForms::Stream& p = s->forms->elem_pair();
+        if (take_pairs(p, eio)) {
+            v = p.v;
+            G = p.G;
+            max_blocks = p.max_blocks;
+        }
     }
     const int64_t want = (eio.nsys + G - 1) / G;
     const int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, max_blocks));
     eio.groups = G;
     v->launch(dim3((unsigned)grid), dim3(v->threads(G)), v->smem_bytes(G, eio.nbuf), stream, nullptr, nullptr, op,
               eio);
-    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, G, v->KL, v->KU, v->SV, s->elem_v->LIN, s->elem_v->LOUT,
+    record_launch(PFSOLVE_KERNEL_STREAMING, v->R, v->W, G, v->KL, v->KU, v->SV, single.v->LIN, single.v->LOUT,
                   v->SCALE, v->PREC, v->ALT, grid, eio.sets ? 2 : 1, 1);
     return true;
 }
@@ -908,13 +987,16 @@ PfSolveResult launch_jw_variant(AppState* s, const JwOperator& op, const JwIO& i
         return PFSOLVE_SUCCESS;
     }
     if (!s->variant) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;  // streaming-only plan
-    AppState::Form f;
+    LaunchForms::Group f;
     f.v = s->variant;
     f.W = s->W;
     f.G = s->G;
     f.max_blocks = s->max_blocks;
-    if (s->dd_few.v && io.nsys <= 3 * (int64_t)s->dd_few.max_blocks * s->dd_few.G) f = s->dd_few;
-    else if (s->dd_many.v) f = s->dd_many;
+    if (s->forms && s->forms->dd) {
+        const LaunchForms::Group& few = s->forms->dd_few();
+        if (few.v && io.nsys <= 3 * (int64_t)few.max_blocks * few.G) f = few;
+        else if (s->forms->dd_many().v) f = s->forms->dd_many();
+    }
     const int64_t want = (io.nsys + f.G - 1) / f.G;
     int64_t grid = std::max<int64_t>(1, std::min<int64_t>(want, f.max_blocks));
     // ALT: a group keeps one parity, so the system step (grid x groups) is even
@@ -1722,14 +1804,7 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
         t.stream_G = cp.stream_G;
         t.stream_max_blocks = cp.stream_max_blocks;
         t.stream_nbuf = cp.stream_nbuf;
-        t.elem_v = cp.elem_v;
-        t.elem_G = cp.elem_G;
-        t.elem_max_blocks = cp.elem_max_blocks;
-        t.elem_nbuf = cp.elem_nbuf;
-        t.stream_pair = cp.stream_pair;
-        t.elem_pair = cp.elem_pair;
-        t.dd_many = cp.dd_many;
-        t.dd_few = cp.dd_few;
+        t.forms = cp.forms.get();
         return launch_jw_variant(&t, op, io, stream);
     }
     AppState t;
@@ -1749,9 +1824,7 @@ PfSolveResult append_chain_fused(PfSolveApplication* dg, const PfSolveLaunchPara
     if (finish_variant(&t, M, LIN, LOUT, SCALE) != PFSOLVE_SUCCESS) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
     sj->chain_plans.push_back(AppState::ChainPlan{KL, KU, L.sv, LIN, LOUT, SCALE, t.variant, t.R, t.W, t.G,
                                                   t.max_blocks, t.stream_v, t.stream_G, t.stream_max_blocks,
-                                                  t.stream_nbuf, t.elem_v, t.elem_G, t.elem_max_blocks,
-                                                  t.elem_nbuf, t.stream_pair, t.elem_pair, t.dd_many,
-                                                  t.dd_few});
+                                                  t.stream_nbuf, t.forms_own});
     return launch_jw_variant(&t, op, io, stream);
 }
 

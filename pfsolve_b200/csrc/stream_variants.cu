@@ -39,9 +39,17 @@ unsigned stream_status_f32mem();
 const StreamVariant* find_stream_variant(int R, int W, int KL, int KU, int SV, int LIN, int LOUT, int SCALE, int PREC,
                                          int ALT, int ELEM)
 {
-    for (auto part : {stream_variants_f64, stream_variants_mixed, stream_variants_alt, stream_variants_f32,
-                      stream_variants_f32mem, stream_elem_f64, stream_elem_mixed, stream_elem_f32,
-                      stream_elem_f32mem, stream_pair_f64, stream_pair_mixed, stream_pair_f32, stream_pair_f32mem}) {
+    // the tables that can hold it: by element copies, in pairs, or neither
+    using Part = const StreamVariant* (*)(int*);
+    static const Part whole[] = {stream_variants_f64, stream_variants_mixed, stream_variants_alt, stream_variants_f32,
+                                 stream_variants_f32mem};
+    static const Part elem[] = {stream_elem_f64, stream_elem_mixed, stream_elem_f32, stream_elem_f32mem,
+                                stream_variants_alt};
+    static const Part pair[] = {stream_pair_f64, stream_pair_mixed, stream_pair_f32, stream_pair_f32mem};
+    const bool pairs = LIN == LAY_XXII && LOUT == LAY_XXII;
+    const Part* parts = pairs ? pair : (ELEM ? elem : whole);
+    for (int p = 0; p < (pairs ? 4 : 5); ++p) {
+        const Part part = parts[p];
         int n = 0;
         const StreamVariant* vs = part(&n);
         for (int i = 0; i < n; ++i) {
