@@ -253,7 +253,9 @@ typedef struct {
 
     /* --- extensions (0 keeps the reference behaviour) --- */
     int mixedPrecisionRefinement; /* 1..3 with doublePrecision: FP32 factor-solve plus this many
-                                     FP64 residual refinement sweeps, FP64 storage (0: plain FP64) */
+                                     FP64 residual refinement sweeps, FP64 storage (0: plain FP64).  Steps
+                                     of 2049..4096 rows run on the streaming kernel alone (full output
+                                     window) */
     int rowsPerThread;            /* 0: autotuned; else 2, 4, 8, 16 or 32 (32: streaming kernel only) */
     int kernelPath;               /* 0: streaming kernel wherever a launch allows it, else the group
                                      kernel (long systems: two passes, with the single pass for
@@ -371,7 +373,9 @@ PFSOLVE_API PfSolveResult PfSolveAppendChain(PfSolveApplication** apps, PfSolveL
  * Three kernels: the group kernel (a group of warps per system, rowsPerThread
  * rows per thread), the streaming solve for real systems (a CTA per item, its
  * table built once; the default for real systems of at most 2048 rows without
- * accumulation, 1024 for the mixed mode's 3-band matvec with an upper solve) and the sweep kernel (one complex system per lane, its
+ * accumulation -- 1024 for the mixed mode's 3-band matvec with an upper solve --
+ * unless so many entries hold so few systems that the table builds would be
+ * most of the time) and the sweep kernel (one complex system per lane, its
  * rows in sequence, a warp per item of 32 systems).  sweepRows = 8 or 16
  * asks for the sweep kernel with that many rows per staged chunk
  * (PFSOLVE_ERROR_UNSUPPORTED_COMBINATION where the batch does not allow it).

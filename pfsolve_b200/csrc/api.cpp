@@ -279,10 +279,10 @@ void LaunchForms::choose_pair(const StreamVariant* v, Stream& out)
     if (p && stream_groups(p, nbuf_req, num_sms, &out.G, &out.nbuf, &out.max_blocks)) out.v = p;
 }
 
-// The streaming kernel with element copies for a plan that has a group-kernel
-// variant: launches whose rows no tensor map describes (odd strides or
-// offsets, row counts that the rows per thread do not divide) take it instead
-// of the group kernel.  The shortest compiled capacity that holds M rows: 4,
+// The streaming kernel with element copies: launches whose rows no tensor map
+// describes (odd strides or offsets, row counts that the rows per thread do not
+// divide) take it instead of the group kernel, or, beyond the group kernel's
+// compiled rows (the mixed mode's 2 048), for want of one.  The shortest compiled capacity that holds M rows: 4,
 // 8, then 16 rows per thread of one warp, 16 of two and four warps, 32 of four.
 void LaunchForms::choose_elem()
 {
@@ -697,10 +697,9 @@ PfSolveResult finish_variant(AppState* s, int64_t M, int LIN, int LOUT, int SCAL
     // systems, a cluster plan), whose launches need buffers those kernels can
     // take.
     s->variant = nullptr;
-    if (choose_stream(s, M, LIN, LOUT, SCALE)) {
-        set_forms(s, M, LIN, LOUT, SCALE);
-        return PFSOLVE_SUCCESS;
-    }
+    const bool tensor = choose_stream(s, M, LIN, LOUT, SCALE);
+    if (M <= kMaxRows) set_forms(s, M, LIN, LOUT, SCALE);
+    if (tensor || (s->forms && s->forms->elem().v)) return PFSOLVE_SUCCESS;
     if (M > kMaxRows && choose_long(s, M, LIN, LOUT, SCALE)) return PFSOLVE_SUCCESS;
     if (M > kMaxRows && choose_cluster(s, M, LIN, LOUT, SCALE)) return PFSOLVE_SUCCESS;
     // nothing compiled fits: distinguish "too long" from "not compiled"
@@ -1468,6 +1467,14 @@ PfSolveResult PfSolveGetShape(const PfSolveApplication* app, int* streaming, int
         if (rowsPerThread) *rowsPerThread = s->cluster_v->R;
         if (warpsPerSystem) *warpsPerSystem = s->cluster_v->W * s->cluster_v->C;
         if (groupsPerCTA) *groupsPerCTA = 1;
+        return PFSOLVE_SUCCESS;
+    }
+    if (!s->stream_v && !s->variant && s->forms && s->forms->elem().v) {  // element copies only
+        const LaunchForms::Stream& f = s->forms->elem();
+        if (streaming) *streaming = 1;
+        if (rowsPerThread) *rowsPerThread = f.v->R;
+        if (warpsPerSystem) *warpsPerSystem = f.v->W;
+        if (groupsPerCTA) *groupsPerCTA = f.G;
         return PFSOLVE_SUCCESS;
     }
     const bool sm = s->stream_v != nullptr;
