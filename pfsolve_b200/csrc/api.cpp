@@ -287,7 +287,7 @@ void LaunchForms::choose_pair(const StreamVariant* v, Stream& out)
 void LaunchForms::choose_elem()
 {
     if (!streams || (alt && prec != PREC_F64)) return;
-    static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 2}, {32, 4}};
+    static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 4}};
     for (const auto& rw : shapes) {
         if (32 * (int64_t)rw[0] * rw[1] < M || (R_req && rw[0] != R_req)) continue;
         const StreamVariant* v = find_stream_variant(rw[0], rw[1], KL, KU, sv, LIN, LOUT, SCALE, prec, alt, 1);

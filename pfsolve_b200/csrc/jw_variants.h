@@ -97,7 +97,6 @@ const StreamVariant* find_stream_variant(int R, int W, int KL, int KU, int SV, i
                                         int PREC, int ALT = 0, int ELEM = 0);
 // Tensor maps of a launch's input and output rows; false when the buffers'
 // alignment, strides or M do not allow the streaming layout.
-bool encode_stream_maps(const StreamVariant* v, const StreamIO& io, CUtensorMap* in, CUtensorMap* out);
 // es: bytes per stored value (8: FP64, 4: FP32); sets: StreamIO::sets.
 bool encode_row_maps(int R, int LIN, int LOUT, int IB, int IBO, const JwIO& io, CUtensorMap* in, CUtensorMap* out,
                      int es = 8, int64_t sets = 0);

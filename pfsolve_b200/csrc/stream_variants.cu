@@ -188,11 +188,6 @@ bool encode_batch_seq_maps(const JwIO& io, BatchSeqEntry* e)
     return true;
 }
 
-bool encode_stream_maps(const StreamVariant* v, const StreamIO& io, CUtensorMap* in, CUtensorMap* out)
-{
-    return encode_row_maps(v->R, v->LIN, v->LOUT, v->IB, v->IBO, io, in, out, prec_f32_storage(v->PREC) ? 4 : 8, io.sets);
-}
-
 unsigned stream_status_fetch_clear()
 {
     const unsigned a = stream_status_f64(), b = stream_status_mixed(), c = cluster_status_fetch_clear();
