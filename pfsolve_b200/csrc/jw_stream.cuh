@@ -150,11 +150,23 @@ struct StCfg {
 // room for fewer than 256 threads' groups, further warps are launched that
 // only help to build it (a table of 4 096 tridiagonal rows took 128 threads
 // 40 us, 32 rows each) and exit before the first solve.  ALT builds two
-// tables in turn and keeps to its groups.
+// tables in turn and keeps to its groups.  The factorisation's scan exchanges
+// through the table and the scratch behind it (st_prologue), and the barriers
+// come next: no more warps than have room there.
+constexpr size_t kScanBytesPerWarp = kScratchPerWarp * sizeof(double);
 template <class C>
 __host__ __device__ constexpr int st_threads(int G)
 {
-    return (C::T * G >= 256 || C::ALT) ? C::T * G : C::kMaxThreads;
+    const int room = 32 * (int)(C::TBL / kScanBytesPerWarp + (size_t)G * C::W);
+    if (C::T * G >= 256 || C::ALT) return C::T * G;
+    return C::kMaxThreads < room ? C::kMaxThreads : room;
+}
+template <class C>
+constexpr bool st_scan_fits()
+{
+    for (int G = 1; G <= 15; ++G)
+        if (st_threads<C>(G) / 32 * kScanBytesPerWarp > C::TBL + (size_t)G * C::W * kScanBytesPerWarp) return false;
+    return true;
 }
 
 // NB: staging buffers per group (2..kStMaxBuffers).

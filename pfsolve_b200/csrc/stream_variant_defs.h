@@ -19,6 +19,7 @@ inline size_t st_smem_fn(int G, int NB)
 template <class C>
 inline int st_threads_fn(int G)
 {
+    static_assert(st_scan_fits<C>(), "the scan's exchange stays clear of the barriers");
     return st_threads<C>(G);
 }
 
