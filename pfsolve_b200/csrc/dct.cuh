@@ -203,7 +203,8 @@ __device__ __forceinline__ void dct_stage(double2* buf, int Ns, int j, const dou
 // One buffer of N complex values per pair; each thread keeps the next pair's
 // 2 N/TPS input values in registers, loaded while the current pair is
 // transformed; type 3 reads X_{N-k} when the pair's turn comes, from L1 (as
-// X_k it was another thread's a moment ago).
+// X_k it was another thread's a moment ago), in rows of up to 32 points from
+// that thread.
 template <int LOGN, int TYPE>
 __global__ void __launch_bounds__(DctShape<LOGN>::NT, DctShape<LOGN>::NT <= 256 ? 2 : 1)
     dct_kernel(const DctIO io, const double2* __restrict__ tw, const double2* __restrict__ pt)
@@ -258,11 +259,26 @@ __global__ void __launch_bounds__(DctShape<LOGN>::NT, DctShape<LOGN>::NT <= 256 
             const bool l1 = y1 < io.nsys, l2 = y2 < io.nsys;
             const double* x1 = io.in + io.in_off + (l1 ? y1 : 0) * io.in_stride;
             const double* x2 = io.in + io.in_off + (l2 ? y2 : 0) * io.in_stride;
+            // X_{N-k}, k = j + i TPS: thread 0's own point 8 - i, else point 7 - i of
+            // thread TPS - j.  Up to 32 points a row it comes from there: rows that
+            // short make the reads of it from L1 below too many for what they fetch
+            // (8 388 608 rows of 8: 789 us with them).
+            constexpr bool kShort = TPS <= 4;
+            const int peer = (int)(threadIdx.x & 31) - j + ((TPS - j) & (TPS - 1));
 #pragma unroll
             for (int i = 0; i < PER; ++i) {
                 const int k = j + i * TPS;
-                // X_{N-k}: loaded for another thread a moment ago (in L1)
-                const double r1 = (k > 0 && l1) ? x1[N - k] : 0.0, r2 = (k > 0 && l2) ? x2[N - k] : 0.0;
+                double r1, r2;
+                if constexpr (kShort) {
+                    const double q1 = TPS > 1 ? __shfl_sync(0xffffffffu, p1[7 - i], peer) : 0.0;
+                    const double q2 = TPS > 1 ? __shfl_sync(0xffffffffu, p2[7 - i], peer) : 0.0;
+                    r1 = j > 0 ? q1 : (i > 0 ? p1[(8 - i) & 7] : 0.0);
+                    r2 = j > 0 ? q2 : (i > 0 ? p2[(8 - i) & 7] : 0.0);
+                } else {
+                    // loaded for another thread a moment ago (in L1)
+                    r1 = (k > 0 && l1) ? x1[N - k] : 0.0;
+                    r2 = (k > 0 && l2) ? x2[N - k] : 0.0;
+                }
                 const double2 c = __ldg(&pt[k]);
                 // z_k = e^{-i t} (X_k + i X_{N-k}) = (X_k cos t + X_{N-k} sin t) + i (X_{N-k} cos t - X_k sin t)
                 const double z1r = __fma_rn(p1[i], c.x, r1 * c.y), z1i = __fma_rn(r1, c.x, -(p1[i] * c.y));
