@@ -81,8 +81,18 @@ struct LaunchForms {
     }
     const Group& dd_many()
     {
-        once(16, [this] { choose_dd(M <= 128 ? 4 : (M <= 256 ? 8 : 16), 1, dd_many_); });
+        once(16, [this] {
+            const bool one_band = sv != SV_TRI && KL + KU == 0;
+            choose_dd(M <= 128 ? 4 : (M <= 256 || (one_band && M >= 520 && M <= 768) ? 8 : 16), 1, dd_many_);
+        });
         return dd_many_;
+    }
+    // Systems that the form for few solves (dd_few: G groups of max_blocks CTAs)
+    int64_t dd_few_systems()
+    {
+        if (sv == SV_NONE && M > 512) return INT64_MAX;
+        const Group& few = dd_few();
+        return (sv != SV_TRI && M > 512 ? 10 : 3) * (int64_t)few.max_blocks * few.G;
     }
 
 private:
@@ -625,11 +635,20 @@ PfSolveResult plan_alt(AppState* s, const PfSolveConfiguration& c, int base_prec
 // Double-double launches of a table-form plan whose rows per thread the caller
 // left open.  Many systems: the table form with the shortest capacity that
 // holds M rows -- 4, 8 and 16 rows per thread of one warp, 16 of two (2^23
-// rows: N = 33 1 361 us at 16 rows of one warp, 461 at 4; 128 383 and 133;
-// 256 205 and 115 at 8; 700 254 at 8 rows of four warps, 182 at 16 of two;
-// 1 000 174 and 140).  Up to three rounds of its resident groups: the register
-// form at 4 rows per thread, whose prologue and solve are the shortest (8
-// systems: N = 512 13.5 against 22.8 us, 1 000 17.7 against 24).
+// rows, against the plan's own shape -- 16 rows per thread of one warp, 8 of
+// more -- before its tables were built by all threads: N = 33 1 364 -> 457 us, 128
+// 418 -> 134, 256 250 -> 118, 700 309 -> 177, 1 000 233 -> 139; of the same
+// build, 205 -> 115 at N = 256, 254 -> 182 at 700, 174 -> 140 at 1 000).  Up to
+// three rounds of its resident groups: the register form at 4 rows per thread,
+// whose prologue and solve are the shortest (8 systems: N = 512 13.5 against
+// 22.8 us, 1 000 17.7 against 24).
+// Kinds other than the tridiagonal one beyond 512 rows, where 16 rows of two warps
+// leave lanes idle and the register form's coefficients are fewer: one-band
+// solves of 520 to 768 rows take the table form of 8 rows and three warps (6 990
+// systems of 600 rows, FP64 storage: 59.7 us, 66.4 with 16; below 520 the edge of
+// one warp's 512 keeps the form that is tested there); the register form
+// serves up to ten rounds (1 349 of 777, two bands: 30 to 32 against 33.8), and every
+// launch of a kind without a solve (13 981 of 600: 46 to 54 us, 79 with 16 rows).
 void LaunchForms::choose_dd(int R, int tbl, Group& f)
 {
     const int64_t W = (M + 32 * (int64_t)R - 1) / (32 * (int64_t)R);
@@ -993,7 +1012,7 @@ PfSolveResult launch_jw_variant(AppState* s, const JwOperator& op, const JwIO& i
     f.max_blocks = s->max_blocks;
     if (s->forms && s->forms->dd) {
         const LaunchForms::Group& few = s->forms->dd_few();
-        if (few.v && io.nsys <= 3 * (int64_t)few.max_blocks * few.G) f = few;
+        if (few.v && io.nsys <= s->forms->dd_few_systems()) f = few;
         else if (s->forms->dd_many().v) f = s->forms->dd_many();
     }
     const int64_t want = (io.nsys + f.G - 1) / f.G;
@@ -2250,9 +2269,9 @@ PfSolveResult batch_configure_stream(PfSolveBatch* b, bool always)
     best_cut(b, spi, stream_us);
     // Many entries of few systems: the items of an SM run one after another,
     // each behind its table build, while the group kernel builds eight an SM at
-    // once.  1 500 entries of one system of 200 rows: 76.8 us here, 25.4 on the
-    // group kernel (bidiagonal 37.6 and 18.9); 400 of 500 rows 29.4 and 17.2;
-    // 64 of 300 systems of 40 rows 23.5 and 58.6.  The estimates' own errors are
+    // once.  1 500 entries of one system of 200 rows: 76.5 us here, 25.6 on the
+    // group kernel (bidiagonal 37.5 and 15.0); 400 of 500 rows 29.4 and 17.5;
+    // 64 of 300 systems of 40 rows 23.3 and 56.2.  The estimates' own errors are
     // the reason for the factor.
     if (!always && group_kernel_us(b) < 0.85 * stream_us) return PFSOLVE_ERROR_UNSUPPORTED_COMBINATION;
     std::vector<double> us;
