@@ -359,7 +359,7 @@ __global__ void __launch_bounds__(256) jw_dd_kernel(const JwOperator op, const D
 // jw_dd_kernel keeps each thread's coefficients in registers, which holds it
 // at 4 or 8 rows per thread, and recomputes per system the chunk products of
 // the solve bands and the scans' multipliers.  None of them depend on the
-// right-hand side: here group 0 builds them once per CTA into shared memory
+// right-hand side: here a CTA's threads build them once into shared memory
 // (the coefficients row by row, so no thread holds a chunk's worth), and every
 // system then costs per row one double-double multiply-add for the local
 // recurrence and one for the coupling, in each direction, plus the matvec.

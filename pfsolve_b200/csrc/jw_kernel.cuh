@@ -885,8 +885,13 @@ __device__ __forceinline__ void jw_run_systems(const JwOperator& op, const JwIO&
     cp_async_wait<0>();
 }
 
+// Matvec-only kinds at 4 rows per thread: two CTAs of 256 threads an SM are
+// enough, so that the compiler takes the registers (110; left to itself 58 to
+// 64, and 65 536 x 512 with three bands took 143.7 us against 137.7).
 template <class C>
-__global__ void __launch_bounds__(C::kMaxThreads) jw_step_kernel(const JwOperator op, const JwIO io, const int W)
+constexpr int kStepCtas = (C::kSV == SV_NONE && C::kR == 4 && C::kMaxThreads == 256) ? 2 : 0;
+template <class C>
+__global__ void __launch_bounds__(C::kMaxThreads, kStepCtas<C>) jw_step_kernel(const JwOperator op, const JwIO io, const int W)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     using TS = typename C::TS;
@@ -940,7 +945,7 @@ __global__ void __launch_bounds__(C::kMaxThreads) jw_step_kernel(const JwOperato
 // through two alternating shared slots, one barrier per fetch.
 // Two CTAs an SM where the coefficients and the data fit 128 registers with hardly
 // a spill: 4 rows per thread, and 8 of a one-band, one-sided FP64 solve (1 500
-// entries of one 2 000-row system: 93.8 us with two, 104.8 with one at 223).
+// entries of one 2 000-row system: 70.6 us with two, 104.8 with one at 223).
 template <class C>
 constexpr int kBatchCtas =
     (C::kR <= 4 || (C::kR <= 8 && C::NB == 1 && C::kSV != SV_TRI && !C::kMixed && !C::kCplx)) ? 2 : 1;

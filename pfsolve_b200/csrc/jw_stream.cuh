@@ -264,8 +264,11 @@ __device__ __forceinline__ int swz_row(int t)
 // are in flight meanwhile), and small batches pay little else, so it is kept
 // short: the bands' loads in blocks ahead of the dependent chains, one division
 // a pivot, cheap band positions and renormalisations, and a logarithmic scan
-// over the warps.  A tridiagonal launch of 8 systems took 16.7 us at N = 512,
-// 26.5 at 2 048 and 87.9 at 4 096 before that, and takes 8.5, 13.7 and 45.3.
+// over the warps; small CTAs launch helper warps for it (st_threads).  Back to
+// back, a tridiagonal launch of 8 systems took 18.6 us at N = 512, 28.8 at 2 048
+// and 89.9 at 4 096 before that, and takes 10.4, 16.4 and 27.0.  (A pivot is
+// 1 - (a c)(1 / d) where it was 1 - (a c) / d: one rounding more for one division
+// less.)
 // Plane p, row i = R*tt + j (tt: thread of a group) is the double at
 // [((p*U + j/2)*T + tt)*2 + (j&1)]: thread tt reads rows 2u, 2u+1 of a plane
 // as one 16-byte word, lanes on consecutive words.
@@ -1292,8 +1295,13 @@ __device__ __forceinline__ void st_kernel(const JwOperator& op, const StreamIO& 
     ld.finish();
 }
 
+// Two CTAs an SM for matvec-only kinds on FP32 storage with FP64 arithmetic at 16
+// rows per thread, whose tables and staging leave room for them: 64 registers
+// (left to itself the compiler takes 72 to 110; 16 000 x 2 000 57.6 -> 49.8 us).
 template <class C>
-__global__ void __launch_bounds__(C::kMaxThreads) jw_stream_kernel(const __grid_constant__ CUtensorMap tm_in,
+constexpr int kStreamCtas = (C::SV == SV_NONE && C::F32MEM && !C::F32 && C::R == 16) ? 2 : 0;
+template <class C>
+__global__ void __launch_bounds__(C::kMaxThreads, kStreamCtas<C>) jw_stream_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                                   const __grid_constant__ CUtensorMap tm_out,
                                                                   const JwOperator op, const StreamIO io)
 {
