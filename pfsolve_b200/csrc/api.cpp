@@ -106,6 +106,7 @@ private:
         cudaGetLastError();
         have.fetch_or(bit, std::memory_order_release);
     }
+    bool elem_pays(int R, int W) const;
     void choose_elem();
     void choose_pair(const StreamVariant* v, Stream& out);
     void choose_dd(int R, int tbl, Group& out);
@@ -294,12 +295,32 @@ void LaunchForms::choose_pair(const StreamVariant* v, Stream& out)
 // divide) take it instead of the group kernel, or, beyond the group kernel's
 // compiled rows (the mixed mode's 2 048), for want of one.  The shortest compiled capacity that holds M rows: 4,
 // 8, then 16 rows per thread of one warp, 16 of two and four warps, 32 of four.
+// Not every shape: complex and ALT variants start at larger capacities than the
+// group kernel's, which pads less (its 4 rows per thread of one warp hold 128
+// rows).  Ratios of this kernel's time to that one's, batches that fill the chip:
+//  * complex, 512 rows of one warp: 33 rows 2.2, 127 1.7 to 2.4, 129 to 255
+//    1.0 (a band or a tridiagonal solve; 3-band upper solve 1.2, on FP32 storage
+//    with FP64 arithmetic 1.0), 257 0.7 to 0.9;
+//  * complex, 1 024 rows of two: the 3-band upper solve in FP64 1.0 to 1.3
+//    throughout; tridiagonal FP64 1.05 to 1.09 up to 704 rows, then 0.8;
+//  * ALT, 2 048 rows of four warps: up to 1 280 rows 1.0 to 1.2; 4 096 rows: 1.15
+//    to 1.5 up to 3 072 rows, 0.9 to 1.1 beyond (and see launch_elem).
+bool LaunchForms::elem_pays(int R, int W) const
+{
+    const int64_t capacity = 32 * (int64_t)R * W;
+    if (alt) return capacity == 4096 ? M > 3584 : (capacity != 2048 || M > 1280);
+    if (LIN == LAY_REAL) return true;
+    if (W == 1) return M > (sv == SV_TRI || prec == PREC_F64_F32MEM ? 128 : 256);
+    return prec != PREC_F64 || (sv == SV_TRI && M > 704);
+}
+
 void LaunchForms::choose_elem()
 {
     if (!streams || (alt && prec != PREC_F64)) return;
     static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 4}};
     for (const auto& rw : shapes) {
         if (32 * (int64_t)rw[0] * rw[1] < M || (R_req && rw[0] != R_req)) continue;
+        if (!R_req && !elem_pays(rw[0], rw[1])) return;
         const StreamVariant* v = find_stream_variant(rw[0], rw[1], KL, KU, sv, LIN, LOUT, SCALE, prec, alt, 1);
         if (v && stream_groups(v, nbuf_req, num_sms, &elem_.G, &elem_.nbuf, &elem_.max_blocks)) {
             elem_.v = v;
@@ -964,6 +985,9 @@ bool launch_elem(AppState* s, const JwOperator& op, const JwIO& io, cudaStream_t
     eio.unit16 = in0 % 16 == 0 && (io.in_stride * es) % 16 == 0 &&
                  (packed || (out0 % 16 == 0 && (io.out_stride * es) % 16 == 0));
     int G = single.G, max_blocks = single.max_blocks;
+    // ALT row sets at 32 rows per thread: two long tables before the first solve
+    // (4 095 rows: 4 rounds 1.1 to 1.9 of the group kernel's time, 16 rounds 0.9 to 1.1)
+    if (v->ALT && v->R == 32 && s->variant && eio.nsys < 8 * (int64_t)max_blocks * G) return false;
     if (eio.nsys >= 4 * (int64_t)s->num_sms) {
         const LaunchForms::Stream& p = s->forms->elem_pair();
         if (take_pairs(p, eio)) {
