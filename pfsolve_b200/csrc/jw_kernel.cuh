@@ -887,9 +887,14 @@ __device__ __forceinline__ void jw_run_systems(const JwOperator& op, const JwIO&
 
 // Matvec-only kinds at 4 rows per thread: two CTAs of 256 threads an SM are
 // enough, so that the compiler takes the registers (110; left to itself 58 to
-// 64, and 65 536 x 512 with three bands took 143.7 us against 137.7).
+// 64): 65 536 x 512 with three bands 143.7 -> 115.8 us.  Upper solves with a band
+// below at 8 rows per thread: at most the 128 registers that a second CTA leaves
+// (2 396 ALT row sets of 3 501 rows 60.8 us with two, 69.1 with one).
 template <class C>
-constexpr int kStepCtas = (C::kSV == SV_NONE && C::kR == 4 && C::kMaxThreads == 256) ? 2 : 0;
+constexpr int kStepCtas = C::kMaxThreads != 256 ? 0
+                          : C::kSV == SV_NONE   ? (C::kR == 4 ? 2 : 0)
+                          : C::kSV == SV_UPPER && C::NB > 1 && C::kR == 8 && !C::kMixed && !C::kF32 && !C::kCplx ? 2
+                                                                                                                   : 0;
 template <class C>
 __global__ void __launch_bounds__(C::kMaxThreads, kStepCtas<C>) jw_step_kernel(const JwOperator op, const JwIO io, const int W)
 {

@@ -1299,7 +1299,7 @@ __device__ __forceinline__ void st_kernel(const JwOperator& op, const StreamIO& 
 // rows per thread, whose tables and staging leave room for them: 64 registers
 // (left to itself the compiler takes 72 to 110; 16 000 x 2 000 57.6 -> 49.8 us).
 template <class C>
-constexpr int kStreamCtas = (C::SV == SV_NONE && C::F32MEM && !C::F32 && C::R == 16) ? 2 : 0;
+constexpr int kStreamCtas = C::SV == SV_NONE && C::F32MEM && !C::F32 && C::R == 16 ? 2 : 0;
 template <class C>
 __global__ void __launch_bounds__(C::kMaxThreads, kStreamCtas<C>) jw_stream_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                                   const __grid_constant__ CUtensorMap tm_out,
