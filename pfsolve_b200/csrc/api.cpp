@@ -303,13 +303,15 @@ void LaunchForms::choose_pair(const StreamVariant* v, Stream& out)
 //    with FP64 arithmetic 1.0), 257 0.7 to 0.9;
 //  * complex, 1 024 rows of two: the 3-band upper solve in FP64 1.0 to 1.3
 //    throughout; tridiagonal FP64 1.05 to 1.09 up to 704 rows, then 0.8;
+//  * real, a caller's 32 rows per thread: four warps alone are compiled (500 rows
+//    1.6 to 6.6);
 //  * ALT, 2 048 rows of four warps: up to 1 280 rows 1.0 to 1.2; 4 096 rows: 1.15
 //    to 1.5 up to 3 072 rows, 0.9 to 1.1 beyond (and see launch_elem).
 bool LaunchForms::elem_pays(int R, int W) const
 {
     const int64_t capacity = 32 * (int64_t)R * W;
     if (alt) return capacity == 4096 ? M > 3584 : (capacity != 2048 || M > 1280);
-    if (LIN == LAY_REAL) return true;
+    if (LIN == LAY_REAL) return R < 32 || M > 2048;
     if (W == 1) return M > (sv == SV_TRI || prec == PREC_F64_F32MEM ? 128 : 256);
     return prec != PREC_F64 || (sv == SV_TRI && M > 704);
 }
@@ -320,7 +322,7 @@ void LaunchForms::choose_elem()
     static const int shapes[][2] = {{4, 1}, {8, 1}, {16, 1}, {16, 2}, {16, 4}, {32, 4}};
     for (const auto& rw : shapes) {
         if (32 * (int64_t)rw[0] * rw[1] < M || (R_req && rw[0] != R_req)) continue;
-        if (!R_req && !elem_pays(rw[0], rw[1])) return;
+        if (!elem_pays(rw[0], rw[1])) return;
         const StreamVariant* v = find_stream_variant(rw[0], rw[1], KL, KU, sv, LIN, LOUT, SCALE, prec, alt, 1);
         if (v && stream_groups(v, nbuf_req, num_sms, &elem_.G, &elem_.nbuf, &elem_.max_blocks)) {
             elem_.v = v;

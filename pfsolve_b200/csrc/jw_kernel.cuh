@@ -889,7 +889,7 @@ __device__ __forceinline__ void jw_run_systems(const JwOperator& op, const JwIO&
 // enough, so that the compiler takes the registers (110; left to itself 58 to
 // 64): 65 536 x 512 with three bands 143.7 -> 115.8 us.  Upper solves with a band
 // below at 8 rows per thread: at most the 128 registers that a second CTA leaves
-// (2 396 ALT row sets of 3 501 rows 60.8 us with two, 69.1 with one).
+// (2 396 ALT row sets of 3 501 rows 53.4 us with two, 69.1 with one).
 template <class C>
 constexpr int kStepCtas = C::kMaxThreads != 256 ? 0
                           : C::kSV == SV_NONE   ? (C::kR == 4 ? 2 : 0)

@@ -78,3 +78,28 @@ def test_alt_row_sets(M, B, kernel):
             outs.append(x)
             app.close()
         assert _agree(outs[0], outs[1], "f64")
+
+
+@pytest.mark.parametrize("M,rows,kernel", [(500, 32, GROUP), (1000, 32, GROUP), (2047, 32, GROUP), (2049, 32, STREAMING),
+                                           (501, 16, STREAMING), (255, 8, STREAMING), (257, 8, GROUP),
+                                           (127, 4, STREAMING), (129, 4, GROUP)])
+def test_rows_per_thread(M, rows, kernel):
+    """A caller's rows per thread, where one of the compiled shapes of that many
+    fits the system."""
+    import torch
+
+    from pfsolve_b200.api import App, last_launch
+    B = (1 << 22) // M
+    x0 = torch.randn(M * B, dtype=torch.float64, device="cuda", generator=torch.Generator(device="cuda").manual_seed(M))
+    bands = torch.from_numpy(WL.permute_bands(J.random_bands(np.random.default_rng(M), M, 2), M)).cuda()
+    outs = []
+    for r in (rows, 0):
+        x = x0.clone()
+        app = App(buffer=bands, outputBuffer=x, M_size=M, size=(M, B), upperBanded=2, jw_type=13, scaleC=1.0,
+                  doublePrecision=1, rowsPerThread=r)
+        app.append()
+        torch.cuda.synchronize()
+        assert last_launch()["kernel"] == (kernel if r else STREAMING), (M, r)
+        outs.append(x)
+        app.close()
+    assert _agree(outs[0], outs[1], "f64")
