@@ -35,6 +35,10 @@ __host__ __device__ constexpr int seq_buf_bytes(int CH) { return CH * 32 * 8; }
 // threads per CTA: 24 warps (85 registers a thread) for K <= 4 with 8-row
 // boxes, else 16 warps (128 registers; 16-row boxes leave shared memory for
 // about 12 warps anyway)
+// The kernel's bound names one CTA an SM, which is all its grid ever has:
+// without it the compiler kept ascending solves of two steps (three without a
+// matvec) to 64 registers for a second CTA, with spills (100-row systems, two
+// steps: 60 000 took 18.8 us and take 16.8, 113 664 took 33.1 and take 31.3).
 template <int K, int CH>
 struct SeqThreads {
     static constexpr int v = (K > 4 || CH > 8) ? 512 : 768;
@@ -73,7 +77,7 @@ __device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, int x, int 
 // and the step that applies the matvec diagonal -- the first for UB 1, the
 // last for UB 0 -- is known at compile time).  CH: rows per box (8 or 16).
 template <int UB, bool MV, bool SV, int K, int CH>
-__global__ void __launch_bounds__(SeqThreads<K, CH>::v) jw_steps_seq_kernel(const __grid_constant__ CUtensorMap tm_in,
+__global__ void __launch_bounds__(SeqThreads<K, CH>::v, 1) jw_steps_seq_kernel(const __grid_constant__ CUtensorMap tm_in,
                                                                       const __grid_constant__ CUtensorMap tm_out,
                                                                       const __grid_constant__ JwSteps S, const JwIO io,
                                                                       const int NW)
